@@ -34,6 +34,7 @@
 
 #include "mulcore.cuh"
 #include "multhread.cuh"
+#include "multc.cuh"
 #include "mulwarp.cuh"
 
 namespace bi {
@@ -367,8 +368,104 @@ static bi_status mul_thread(const T* a, const T* b, T* r, uint32_t m, uint64_t n
 }
 
 // ---------------------------------------------------------------------------
+// Products of large operands on the tensor cores (multc.cuh), one instance
+// per CTA at a time, the CTAs persistent.  Bound by the tensor core at the
+// large sizes: 65 cycles a matrix instruction of 128 x 128 x 16 digit
+// products (its peak), half of them on the zeros beside the convolution's
+// triangle; 4096 full products of 1024 limbs 0.63 ms (34.7K cycles an
+// instance on the tensor core alone, 44.6K measured), 2.65 ms on the CTA
+// kernel's integer pipe.
+// ---------------------------------------------------------------------------
+__device__ uint32_t tc_gave_up;    // waits on the tensor core that ran out (never seen)
+
+template <typename T, int P>
+__global__ void __launch_bounds__(TcShape<P>::THREADS, 1)
+mul_tc_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ r, uint64_t n, TcGeom g) {
+    extern __shared__ __align__(128) uint8_t smem_tc[];
+    auto limb = [&](const T* p, uint64_t inst, uint32_t x) -> uint64_t {
+        const T* row = p + inst * g.m;
+        if constexpr (sizeof(T) == 8) return row[x];
+        else return row[2 * x] | (2 * x + 1 < g.m ? (uint64_t)row[2 * x + 1] << 32 : 0ull);
+    };
+    tc_products<P>(
+        g, smem_tc, blockIdx.x, gridDim.x, n, &tc_gave_up,
+        [&](uint64_t inst, uint32_t x) { return limb(a, inst, x); },
+        [&](uint64_t inst, uint32_t x) { return limb(b, inst, x); },
+        [&](uint64_t inst, uint32_t x, uint64_t v) {
+            T* row = r + inst * g.out_words;
+            if constexpr (sizeof(T) == 8) {
+                row[x] = v;
+            } else {                          // an odd m leaves the top limbs without words
+                if (2 * x < g.out_words) row[2 * x] = (uint32_t)v;
+                if (2 * x + 1 < g.out_words) row[2 * x + 1] = (uint32_t)(v >> 32);
+            }
+        });
+}
+
+// CTAs an SM holds of a kernel that allocates tensor memory, from its
+// registers, shared memory and accumulator columns (the runtime's occupancy
+// query answers 1 for every such kernel).
+static int tc_ctas_per_sm(const void* kern, uint32_t threads, size_t smem, uint32_t cols) {
+    cudaFuncAttributes at;
+    if (cudaFuncGetAttributes(&at, kern) != cudaSuccess) {
+        cudaGetLastError();                    // not the launch's error
+        return 1;
+    }
+    const int by_regs = 65536 / (((at.numRegs + 7) / 8 * 8) * (int)threads);
+    const int by_smem = (int)(228 * 1024 / (smem + at.sharedSizeBytes + 1024)), by_cols = (int)(512 / cols);
+    return std::max(1, std::min(by_regs, std::min(by_smem, by_cols)));
+}
+
+template <typename T, int P>
+static bi_status mul_tc_launch(const T* a, const T* b, T* r, uint32_t m, uint64_t n, uint32_t L, uint32_t out_limbs,
+                               uint32_t out_words, cudaStream_t st) {
+    TcGeom g = tc_geometry<P>(L, out_limbs);
+    g.m = m;
+    g.out_words = out_words;
+    g.NA = 2;
+    if (TcSmem<P>(g).total > 227 * 1024) g.NA = 1;
+    const size_t smem = TcSmem<P>(g).total;
+    auto kern = mul_tc_kernel<T, P>;
+    cudaError_t e = smem_opt_in((const void*)kern, smem);
+    if (e != cudaSuccess) return set_error(BI_ECUDA, "mul: %s", cudaGetErrorString(e));
+    const uint64_t cap = (uint64_t)num_sms() * tc_ctas_per_sm((const void*)kern, TcShape<P>::THREADS, smem, TcShape<P>::TMEM_COLS);
+    kern<<<(unsigned)(n < cap ? n : cap), TcShape<P>::THREADS, smem, st>>>(a, b, r, n, g);
+    return check_launch("mul tensor kernel");
+}
+
+template <typename T, bool FULL>
+static bi_status mul_tc(const T* a, const T* b, T* r, uint32_t m, uint64_t n, cudaStream_t st) {
+    const uint32_t L = sizeof(T) == 8 ? m : (m + 1) / 2;
+    const uint32_t ol = FULL ? 2 * L : L, ow = FULL ? 2 * m : m;
+    // the narrowest accumulator whose 128 rows hold the product: a matrix
+    // instruction takes 40 / 42 / 49 / 57 / 65 cycles at P = 16 / 32 / 64 / 96
+    // / 128 (A's 4 KB of shared memory a step first, then the tensor core)
+    if (ol <= 16 * 16) return mul_tc_launch<T, 16>(a, b, r, m, n, L, ol, ow, st);
+    if (ol <= 16 * 32) return mul_tc_launch<T, 32>(a, b, r, m, n, L, ol, ow, st);
+    if (ol <= 16 * 64) return mul_tc_launch<T, 64>(a, b, r, m, n, L, ol, ow, st);
+    if (ol <= 16 * 96) return mul_tc_launch<T, 96>(a, b, r, m, n, L, ol, ow, st);
+    return mul_tc_launch<T, 128>(a, b, r, m, n, L, ol, ow, st);
+}
+
+// ---------------------------------------------------------------------------
 
 constexpr uint32_t MUL_MAX_L = 4096;   // u64-view limbs per operand
+
+// Products on the tensor cores: the largest sizes always; down to 33 limbs
+// while a batch is a few CTAs an SM.  Measured against the CTA kernel's best
+// tiling (u64): full products of 192 / 256 / 512 / 1024 / 2048 / 4096 limbs
+// 1.43 / 1.84 / 2.82 / 4.18 / 4.13 / 6.0 times its rate at 2^22 limbs an
+// operand, of 128 limbs 0.95; truncated ones of 250 / 512 / 1024 / 2048 limbs
+// 1.22 / 2.05 / 3.03 / 4.59, of 192 limbs 0.92.  With 8 instances an SM or
+// fewer one instance's serial rows bound the CTA kernel: 64 limbs 4.5 us
+// against 12.7 with one instance, 11.5 against 13.9 with 1216; 1024 limbs
+// 26.9 against 146.
+constexpr uint32_t MUL_TC_MIN_L = 33, MUL_TC_FULL_L = 160, MUL_TC_TRUNC_L = 208, MUL_TC_SM_INSTANCES = 8;
+
+static bool mul_use_tc(uint32_t L, bool full, uint64_t n) {
+    if (L >= (full ? MUL_TC_FULL_L : MUL_TC_TRUNC_L)) return true;
+    return L >= MUL_TC_MIN_L && n <= (uint64_t)MUL_TC_SM_INSTANCES * num_sms();
+}
 constexpr uint32_t MUL_WARP_MAX_L = 32;    // full products above MUL_THREAD_MAX_L up to here: the warp kernel
 
 // ---------------------------------------------------------------------------
@@ -463,6 +560,9 @@ static bi_status mul_launch(const T* a, const T* b, T* r, uint32_t m, uint64_t n
             if constexpr (FULL) return mul_warp<T>(a, b, r, m, n, st);
         }
     }
+    MulTune t;
+    if (mul_use_tc(L, FULL, n) && !mul_tuning_lookup((int)sizeof(T), FULL, L, &t))
+        return mul_tc<T, FULL>(a, b, r, m, n, st);
     return mul_launch_geom<T, FULL>(a, b, r, m, n, mul_geom_for<T, FULL>(L, n), st);
 }
 
@@ -511,7 +611,9 @@ static bi_status mul_chain(const T* a, const T* b, T* r, uint32_t m, uint64_t n,
 // limbs the thread kernel (64-bit limbs, one thread an instance), recorded
 // as {0, 1}, beside the CTA
 // kernel's tilings (64-bit limbs: row_mac8) -- the arithmetic's word width
-// and the threads an instance are part of what is tuned.
+// and the threads an instance are part of what is tuned.  Where the call
+// would go to the tensor cores they are a candidate too: one instance a CTA,
+// {1, 1}, and nothing is recorded when they are the fastest.
 template <typename T, bool FULL>
 static bi_status mul_autotune(const T* a, const T* b, T* r, uint32_t m, uint64_t n, int reps, int* chosen,
                               cudaStream_t st) {
@@ -544,11 +646,17 @@ static bi_status mul_autotune(const T* a, const T* b, T* r, uint32_t m, uint64_t
     float best = 1e30f;
     MulTune pick = {cands[0].first, cands[0].second};
     bi_status st_out = BI_OK;
-    for (const auto& c : cands) {
+    const bool tc = mul_use_tc(L, FULL, n);
+    const size_t ntiled = cands.size();
+    if (tc) cands.push_back({1, 1});
+    bool pick_tc = false;
+    for (size_t ci = 0; ci < cands.size(); ci++) {
+        const auto& c = cands[ci];
+        const bool on_tc = ci >= ntiled;
         std::vector<float> ts;
         for (int k = 0; k <= reps && st_out == BI_OK; k++) {   // the first run warms up
             cudaEventRecord(e0, st);
-            st_out = run(c.first, c.second);
+            st_out = on_tc ? mul_tc<T, FULL>(a, b, r, m, n, st) : run(c.first, c.second);
             cudaEventRecord(e1, st);
             if (cudaEventSynchronize(e1) != cudaSuccess) st_out = set_error(BI_ECUDA, "mul autotune: %s",
                                                                             cudaGetErrorString(cudaGetLastError()));
@@ -562,6 +670,7 @@ static bi_status mul_autotune(const T* a, const T* b, T* r, uint32_t m, uint64_t
         if (med < best) {
             best = med;
             pick = {c.first, c.second};
+            pick_tc = on_tc;
         }
     }
     cudaEventDestroy(e0);
@@ -571,10 +680,12 @@ static bi_status mul_autotune(const T* a, const T* b, T* r, uint32_t m, uint64_t
     cudaGetDevice(&dev);
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tune[std::make_tuple(dev, (int)sizeof(T), FULL ? 1 : 0, L)] = pick;
+        const auto key = std::make_tuple(dev, (int)sizeof(T), FULL ? 1 : 0, L);
+        if (pick_tc) g_tune.erase(key);    // the library's own choice
+        else g_tune[key] = pick;
     }
     // leave r as one plain call with the chosen tiling writes it
-    BI_RETURN_IF(run(pick.ipc, pick.S));
+    BI_RETURN_IF((pick_tc ? mul_tc<T, FULL>(a, b, r, m, n, st) : run(pick.ipc, pick.S)));
     if (chosen) {
         chosen[0] = (int)pick.ipc;
         chosen[1] = (int)pick.S;

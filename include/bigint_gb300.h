@@ -109,14 +109,17 @@ bi_status bi_mulfull_u32(const uint32_t* a, const uint32_t* b, uint32_t* r,
 /* and row slices per window pair. Full products of at most 24 64-bit     */
 /* limbs and truncated ones of at most 32 run by default on the thread    */
 /* kernel (one thread an instance, 64-bit limbs), full products of 25 to  */
-/* 32 limbs on the warp kernel (32-bit words). bi_mul_autotune_* times    */
+/* 32 limbs on the warp kernel (32-bit words); full products of at least  */
+/* 160 limbs, truncated ones of at least 208 and, in small batches, those */
+/* of 33 limbs on run on the tensor cores.  bi_mul_autotune_* times       */
 /* every tiling that fits on the caller's a, b -- and the warp kernel for */
 /* full products of at most 32 64-bit limbs, the thread kernel where it   */
 /* takes the size -- (median of `reps` runs each), records the fastest    */
 /* for this device, limb width, product kind (full != 0: bi_mulfull_*)    */
 /* and m, which later calls then use, and leaves r as that call writes    */
 /* it; synchronous on `stream`.  chosen (may be NULL) gets {instances per */
-/* CTA, slices}, or {0, 0} when the warp kernel was fastest, {0, 1} for   */
+/* CTA, slices} ({1, 1} for the tensor cores too, which stay the default), */
+/* or {0, 0} when the warp kernel was fastest, {0, 1} for                  */
 /* the thread kernel.  The reference fixes its tiling per size at compile */
 /* time (ipb and the Q limbs per thread, cuda/main.cu:15-28).             */
 /* bi_mul_set_tuning_* sets a tiling by hand (BI_EINVAL if it does not    */
