@@ -4,6 +4,7 @@
 // (cuda/main.cu:108-222, 280-419): allocate device buffers, copy the inputs
 // in, launch, copy the result out and free.  Unlike the reference they
 // report every failure as a status code instead of printing and carrying on.
+#include <algorithm>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -70,6 +71,20 @@ cudaError_t smem_opt_in(const void* func, size_t smem) {
     e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) done.push_back({func, dev, smem});
     return e;
+}
+
+// CTAs an SM holds of a kernel that allocates tensor memory, from its
+// registers, shared memory and accumulator columns (the runtime's occupancy
+// query answers 1 for every such kernel).
+int tc_ctas_per_sm(const void* kern, uint32_t threads, size_t smem, uint32_t cols) {
+    cudaFuncAttributes at;
+    if (cudaFuncGetAttributes(&at, kern) != cudaSuccess) {
+        cudaGetLastError();                    // not the launch's error
+        return 1;
+    }
+    const int by_regs = 65536 / (((at.numRegs + 7) / 8 * 8) * (int)threads);
+    const int by_smem = (int)(228 * 1024 / (smem + at.sharedSizeBytes + 1024)), by_cols = (int)(512 / cols);
+    return std::max(1, std::min({by_regs, by_smem, by_cols}));
 }
 
 static bi_status cuda_ok(cudaError_t e, const char* what) {

@@ -32,6 +32,7 @@
 // cost less than a CTA running the steps above (div_use_long holds the
 // measured crossover, which depends on the batch size too).
 #include "divblock.cuh"
+#include "divtc.cuh"
 #include "divcore.cuh"
 #include "divsmall.cuh"
 
@@ -281,6 +282,80 @@ static void launch_div_blk(const T* u, const T* v, T* q, T* r, uint8_t* status, 
     else launch_blk<T, 32, 8, 4>(u, v, q, r, status, mu, mv, n, s);
 }
 
+// ---------------------------------------------------------------------------
+// Long division 31 quotient limbs at a time on the tensor cores (divtc.cuh),
+// one instance a CTA at a time, the CTAs persistent.  2048 divisions of 2048
+// by 1024 limbs 3400 -> 626 us, 8192 of 512 by 256 1013 -> 409: a quotient
+// block's chain -- estimate, product, fold, carries -- is about 6K cycles of
+// latency with four CTAs an SM (issue slots 45 % busy), of which the matrix
+// instructions are 1.1K at 1024 limbs.
+// ---------------------------------------------------------------------------
+template <typename T, int P>
+__global__ void __launch_bounds__(DtShape<P>::NT)
+div_tc_kernel(const T* __restrict__ u, const T* __restrict__ v, T* __restrict__ q, T* __restrict__ r,
+              uint8_t* __restrict__ status, uint64_t n, DtGeom g) {
+    extern __shared__ __align__(128) uint8_t smem_dt[];
+    const DtSmem<P> lay(g);
+    const uint32_t bar = tc_smem_addr(smem_dt) + lay.bar;
+    const uint32_t tmem = tc_alloc<DtShape<P>::TMEM_COLS>(bar + 8, [&] { tc_bar_init(bar, 1); });
+    uint32_t phase = 0;
+    for (uint64_t inst = blockIdx.x; inst < n; inst += gridDim.x) {
+        const T* ui = u + inst * g.mu;
+        const T* vi = v + inst * g.mv;
+        T* qi = q + inst * g.mu;
+        T* ri = r + inst * g.mv;
+        const uint8_t st = dt_divide<P>(
+            g, lay, smem_dt, tmem, phase, [&](uint32_t i) { return limb64(ui, g.mu, i); },
+            [&](uint32_t i) { return limb64(vi, g.mv, i); }, [&](uint32_t i, uint64_t x) { put_limb64(qi, g.mu, i, x); },
+            [&](uint32_t i, uint64_t x) { put_limb64(ri, g.mv, i, x); });
+        if (status && threadIdx.x == 0) status[inst] = st;
+    }
+    tc_free<DtShape<P>::TMEM_COLS>(tmem);
+}
+
+template <typename T, int P>
+static bi_status launch_div_tc(const T* u, const T* v, T* q, T* r, uint8_t* status, uint64_t n, const DtGeom& g,
+                               cudaStream_t s) {
+    const size_t smem = DtSmem<P>(g).total;
+    auto kern = div_tc_kernel<T, P>;
+    cudaError_t e = smem_opt_in((const void*)kern, smem);
+    if (e != cudaSuccess) return set_error(BI_ECUDA, "div: %s", cudaGetErrorString(e));
+    const uint64_t cap = (uint64_t)num_sms() * tc_ctas_per_sm((const void*)kern, DtShape<P>::NT, smem, DtShape<P>::TMEM_COLS);
+    kern<<<(unsigned)(n < cap ? n : cap), DtShape<P>::NT, smem, s>>>(u, v, q, r, status, n, g);
+    return check_launch("div tensor kernel");
+}
+
+// the narrowest accumulator whose rows hold the divisor
+template <typename T>
+static bi_status div_tc(const T* u, const T* v, T* q, T* r, uint8_t* status, uint32_t mu, uint32_t mv, uint64_t n,
+                        cudaStream_t s) {
+    const DtGeom g = dt_geom(mu, mv, (int)sizeof(T));
+    if (g.MV <= (uint32_t)DtShape<16>::MAX_K) return launch_div_tc<T, 16>(u, v, q, r, status, n, g, s);
+    if (g.MV <= (uint32_t)DtShape<32>::MAX_K) return launch_div_tc<T, 32>(u, v, q, r, status, n, g, s);
+    if (g.MV <= (uint32_t)DtShape<48>::MAX_K) return launch_div_tc<T, 48>(u, v, q, r, status, n, g, s);
+    if (g.MV <= (uint32_t)DtShape<64>::MAX_K) return launch_div_tc<T, 64>(u, v, q, r, status, n, g, s);
+    if (g.MV <= (uint32_t)DtShape<80>::MAX_K) return launch_div_tc<T, 80>(u, v, q, r, status, n, g, s);
+    return launch_div_tc<T, 128>(u, v, q, r, status, n, g, s);
+}
+
+// Measured against the lane groups, the warps and the shifted inverse (us, u64,
+// before / on the tensor cores): an instance costs about 8K cycles before its
+// first quotient block (the reciprocal, the divisor's digits), which a batch
+// that fills the GPU earns back above a product of divisor and quotient limbs of
+// some 6000 to 9400 (16384 divisions with 128-limb divisors: 31 quotient limbs
+// 146 / 183, 62 limbs 275 / 246; 4096 with 512: 8 limbs 64 / 80, 16 limbs 93 /
+// 79; 2m by m limbs: m = 80 472 / 485, 100 574 / 472, 256 1013 / 409, 1024
+// 3399 / 626, 2000 6468 / 982).  With few instances the blocks' shorter chain
+// wins from about 20 quotient limbs on: 1 division of 2m by m limbs with m = 40
+// 20 / 13, 64 30 / 15, 256 83 / 26, 1024 360 / 89; 608 of them with m = 40 22 /
+// 18; 2432 with m = 72 61 / 54, with m = 64 50 / 54.
+static bool div_use_tc(uint32_t MU, uint32_t MV, uint64_t n) {
+    const uint64_t ql = MU - MV + 1, sms = (uint64_t)num_sms();
+    if (MV < 40 || MV > (uint32_t)DtShape<128>::MAX_K) return false;
+    if (MV >= 65 && MV * ql >= 9400) return true;
+    return (ql >= 20 && n <= 4 * sms) || (MV >= 65 && ql >= 48 && n <= 16 * sms);
+}
+
 // dividend limbs (u64 view) per instance: any long division, and the shifted inverse's limit
 constexpr uint32_t DIV_MAX_MU64 = 8192, DIV_SHINV_MAX_MU64 = 2048;
 constexpr int DIV_AUTO = 0, DIV_SHINV = 1, DIV_LONG = 2;   // method of div_entry
@@ -306,6 +381,7 @@ static bi_status div_entry(const T* u, const T* v, T* q, T* r, uint8_t* status, 
         launch_div_thread(u, v, q, r, status, mu, mv, n, (cudaStream_t)s);
         return check_launch("div thread kernel");
     }
+    if (method == DIV_AUTO && div_use_tc(g.MU, g.MV, n)) return div_tc(u, v, q, r, status, mu, mv, n, (cudaStream_t)s);
     // the shifted inverse holds its operands in shared memory: dividends above
     // DIV_SHINV_MAX_MU64 limbs always take long division
     if (method != DIV_SHINV && g.MV <= (uint32_t)DIV_LONG_MAX_MV &&

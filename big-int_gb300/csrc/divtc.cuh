@@ -1,0 +1,520 @@
+// divtc.cuh -- long division by medium and large divisors, DT_KB quotient
+// limbs at a time, the quotient block times the divisor on the tensor cores.
+//
+// One CTA divides one instance; the running remainder ("window")
+// lies in shared memory, the divisor as f16 digits in the Toeplitz layout of
+// multc.cuh, written once per instance.  Per block of quotient limbs:
+//   estimate  q^ = the top 32 window limbs times the 32-limb reciprocal of the
+//             divisor's top 32 limbs (Barrett), the upper half of a 32-by-32
+//             limb product over the CTA's threads;
+//   product   q^ V as a digit convolution: q^'s core matrices in shared
+//             memory, then one chain of matrix instructions;
+//   subtract  each thread folds its accumulator row with its window limbs, one
+//             carry lookahead joins the rows;
+//   check     a negative window or one not below the divisor (q^ is at most
+//             one too large, two too small; both take chance 2^-58 or so on
+//             random operands) is corrected with the whole CTA.
+// Digits are balanced, in [-128, 127]: byte k of x + 0x8080..80 less 128.  A
+// column then sums at most 249 products (q^ has 31 limbs and a carry digit) of
+// magnitude 2^14 at most, below 2^22, so that one accumulator holds a whole
+// block exactly and 1.5 2^23 + v has v in its low bits.
+//
+// With W < V B^31, V's top bit set and K >= 32 limbs, Wt and Vh the top 32
+// limbs of W (K + 31 limbs) and V and I = floor((B^64 - 1) / Vh): q^ =
+// floor((floor(Wt (I - B^32) / B^32) + Wt) / B) differs from floor(W / V) by at
+// most one either way, and by one more below for the columns of the product
+// that are left out.  A divisor of fewer than 32 limbs is scaled by B^(32-K),
+// which scales the remainder.
+#pragma once
+
+#include "divsmall.cuh"
+#include "multc.cuh"
+#include "multhread.cuh"
+
+namespace bi {
+
+constexpr int DT_KB = 31;            // quotient limbs a block
+constexpr uint64_t DT_HALF = 0x8080808080808080ull;
+constexpr int DT_MAX_CORRECTIONS = 4;
+
+template <int P>
+struct DtShape {
+    static constexpr int Q = P / 8;                              // limbs a row
+    static constexpr int H = P >= 80 ? 2 : 1;                    // threads a row of the accumulator
+    static constexpr int NT = 128 * H;                           // threads
+    static constexpr int QT = Q / H;                             // limbs a thread
+    static constexpr int T0 = -256;                              // first term: q^'s 249 digits, down to a multiple of 16
+    static constexpr int STEPS = (P - T0) / 16;                  // matrix instructions a block
+    static constexpr int CM = Q + 2 * STEPS - 1;                 // core matrices of q^
+    static constexpr int KMIN = -((-T0 + P - 1) / P);            // row offset of the first term
+    static constexpr int R = ((128 - KMIN) + 6) / 8 * 8 + 1;     // rows of the divisor's image, % 8 == 1
+    static constexpr int MAX_K = 128 * Q - DT_KB - 2;            // divisor limbs: the rows hold K + 33
+    static constexpr uint32_t TMEM_COLS = tc_pow2(P);
+    // Place of window limb x: threads 8 limbs apart would all meet in the same
+    // banks, so that the eight-limb shapes pad one limb after every eight
+    // (1671 -> 988 us for 1048 divisions of 4000 by 2000 limbs; the others ran
+    // 3-5 % slower with it)
+    __host__ __device__ static constexpr int at(int x) { return QT % 8 == 0 ? x + (x >> 3) : x; }
+    static constexpr int QLO = 2 * STEPS - 32, QHI = Q + 1;      // zero limbs below and above q^ that its blocks read
+};
+
+struct DtGeom {
+    uint32_t mu, mv;       // limbs per dividend / divisor in the caller's type
+    uint32_t MU, MV;       // the same in 64-bit limbs
+    uint32_t UL;           // window limbs (places)
+};
+
+template <int P>
+struct DtSmem {
+    uint32_t stage, win, inv, part, qraw, qh, cs, scratch, bar, total;
+    __host__ __device__ explicit DtSmem(const DtGeom& g) {
+        using S = DtShape<P>;
+        stage = S::R * S::Q * 16;
+        win = stage + S::CM * 128;
+        inv = win + g.UL * 8;
+        part = inv + 64 * 8;
+        qraw = part + 3 * S::NT * 8;
+        qh = qraw + (S::QLO + 32 + S::QHI + 1) / 2 * 16;
+        cs = qh + 34 * 8;
+        scratch = cs + (S::NT + 1) * 8;
+        bar = scratch + 3 * 32 * 4;
+        total = bar + 16;
+    }
+};
+
+__host__ __device__ inline DtGeom dt_geom(uint32_t mu, uint32_t mv, int wbytes) {
+    DtGeom g;
+    g.mu = mu;
+    g.mv = mv;
+    g.MU = wbytes == 8 ? mu : (mu + 1) / 2;
+    g.MV = wbytes == 8 ? mv : (mv + 1) / 2;
+    g.UL = (g.MU + 64) * 9 / 8 + 2;
+    g.UL = g.UL / 2 * 2;
+    return g;
+}
+
+// two bytes of w less 128 as a pair of f16 (see tc_digits)
+__device__ __forceinline__ uint32_t dt_digits(uint32_t w, uint32_t sel) {
+    const uint32_t x = __byte_perm(w, 0x64646464u, sel);
+    const __half2 y = __hsub2(*reinterpret_cast<const __half2*>(&x), __half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480)));
+    return *reinterpret_cast<const uint32_t*>(&y);
+}
+
+// x = x + y (sub: x - y) mod B^len for window limbs x from x0 on and y given
+// by limb(i), the whole CTA; returns the carry (borrow) out.
+template <typename S, typename Limb>
+__device__ uint32_t dt_addsub(uint64_t* win, int x0, Limb limb, int len, bool sub, uint32_t* scratch) {
+    constexpr int NT = S::NT;
+    const int per = (len + NT - 1) / NT, lo = min((int)threadIdx.x * per, len), hi = min(lo + per, len);
+    uint32_t c = 0, all = 1;
+    for (int i = lo; i < hi; i++) {      // carries with none in
+        const uint64_t y = limb(i), a = win[S::at(x0 + i)];
+        const uint64_t s = sub ? a - y : a + y;
+        const uint32_t k = sub ? a < y : s < y;
+        const uint64_t t = sub ? s - c : s + c;
+        c = k | (sub ? s < c : t < s);
+        all &= sub ? t == 0 : t == ~0ull;
+    }
+    const uint32_t g = c, p = hi > lo ? (all & !c) : 1u;
+    const uint32_t cin = block_carry_in(g, p, threadIdx.x == 0, scratch);
+    c = cin;
+    for (int i = lo; i < hi; i++) {
+        const uint64_t y = limb(i), a = win[S::at(x0 + i)];
+        const uint64_t s = sub ? a - y : a + y;
+        const uint32_t k = sub ? a < y : s < y;
+        const uint64_t t = sub ? s - c : s + c;
+        c = k | (sub ? s < c : t < s);
+        win[S::at(x0 + i)] = t;
+    }
+    return __syncthreads_or(threadIdx.x == NT - 1 && (hi > lo ? c : cin));
+}
+
+// carry out of each lane's (g, p), carry-in 0: the carry into the lane, and out of lane 31
+__device__ __forceinline__ uint32_t dt_lane_carry(uint32_t g, uint32_t p, uint32_t& cout) {
+    const WarpCarry w = warp_carry_resolve(__ballot_sync(0xffffffffu, g | p), __ballot_sync(0xffffffffu, g), 0);
+    cout = w.cout;
+    return (w.carries >> (threadIdx.x & 31)) & 1u;
+}
+
+// Limb `lane` of sum over lanes t of (lo + mid B + hi B^2) B^t + extra B^t,
+// hi small: the columns of a product and a number added to it, one a lane.
+__device__ __forceinline__ uint64_t dt_fold(uint64_t lo, uint64_t mid, uint64_t hi, uint64_t extra) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint64_t m = __shfl_up_sync(0xffffffffu, mid, 1), h = __shfl_up_sync(0xffffffffu, hi, 2);
+    if (lane < 1) m = 0;
+    if (lane < 2) h = 0;
+    uint64_t sum = lo + m;
+    uint32_t e = sum < m;
+    sum += h;
+    e += sum < h;
+    sum += extra;
+    e += sum < extra;
+    uint32_t ein = __shfl_up_sync(0xffffffffu, e, 1), over;
+    if (lane == 0) ein = 0;
+    sum += ein;
+    return sum + dt_lane_carry(sum < ein, sum == ~0ull, over);
+}
+
+// One step of dt_recip: P limbs of y to 2 P.
+template <int P>
+__device__ __forceinline__ void dt_recip_step(const uint64_t* v, uint64_t* y, uint64_t* t) {
+    const int lane = (int)(threadIdx.x & 31);
+    const uint64_t* V = v + 32 - 2 * P;
+    const uint64_t* Y = y + 32 - P;
+    // column P - 1 + lane of X Y, X's limbs above its top zero, lanes 0 .. P + 1
+    auto column = [&](const uint64_t* X, uint64_t& c0, uint64_t& c1, uint32_t& c2) {
+        c0 = c1 = 0;
+        c2 = 0;
+        if (lane <= P + 1) {
+#pragma unroll
+            for (int i = 0; i < P; i++) mac3(c0, c1, c2, X[P - 1 + lane - i], Y[i]);
+        }
+    };
+    uint64_t c0, c1;
+    uint32_t c2, over;
+    const bool mid = lane >= 1 && lane <= P + 1;
+    column(V, c0, c1, c2);
+    // S = V + V Y / B^P mod B^(P+1) = -E, limb j on lane j + 1; E = B^2P (1 - V x)
+    uint64_t S = dt_fold(c0, c1, c2, mid ? V[lane - 1] : 0);
+    const bool pos = (__shfl_sync(0xffffffffu, S, P + 1) >> 63) == 0;
+    const uint32_t one = dt_lane_carry(lane == 0, lane >= 1 && S == 0, over);
+    if (!pos) S = ~S + one;
+    if (mid) t[lane - 1] = S;
+    __syncwarp();
+    // D = |E| + |E| Y / B^P, limb j on lane j + 1
+    column(t, c0, c1, c2);
+    const uint64_t D = dt_fold(c0, c1, c2, mid ? S : 0);
+    uint64_t dl = __shfl_down_sync(0xffffffffu, D, 1);
+    if (lane > P) dl = 0;
+    // y B^P -+ D, kept within [0, B^2P)
+    const bool in = lane < 2 * P;
+    const uint64_t a = lane >= P && in ? Y[lane - P] : 0;
+    uint64_t r = pos ? a - dl : a + dl;
+    const uint32_t cy = dt_lane_carry(in && (pos ? a < dl : r < dl), in && (pos ? r == 0 : r == ~0ull), over);
+    r = pos ? r - cy : r + cy;
+    // the carry out of lane 2 P - 1 is the carry into lane 2 P (there is none above lane 31)
+    if (2 * P < 32) over = __shfl_sync(0xffffffffu, cy, (2 * P) & 31);
+    if (over) r = pos ? 0 : ~0ull;
+    __syncwarp();
+    if (in) y[32 - 2 * P + lane] = r;
+    __syncwarp();
+}
+
+// y[0..32) = about floor((B^64 - 1) / V) - B^32 for V = v[0..32), top bit set,
+// v[32] = 0, by one warp: Newton's iteration from the top limb's reciprocal,
+// y + 1 = x -> x + x (1 - V x), with 1, 2, .. 16 limbs of y giving twice as
+// many.  The top halves of 1 - V x cancel and the lowest columns are left out:
+// within 2^24 units of the last limb in 3000 random and extreme divisors,
+// which moves a quotient block by one with a chance of 2^-40.  `t`: 34 limbs.
+__device__ __forceinline__ void dt_recip(const uint64_t* v, uint64_t* y, uint64_t* t) {
+    const int lane = (int)(threadIdx.x & 31);
+    t[lane] = 0;
+    if (lane < 2) t[32 + lane] = 0;
+    if (lane == 0) y[31] = recip_limb(v[31]);
+    __syncwarp();
+    dt_recip_step<1>(v, y, t);
+    dt_recip_step<2>(v, y, t);
+    dt_recip_step<4>(v, y, t);
+    dt_recip_step<8>(v, y, t);
+    dt_recip_step<16>(v, y, t);
+}
+
+// One division.  load_u(i) (i < g.MU), load_v(i) (i < g.MV) give limbs,
+// store_q(i, x) for i < g.MU and store_r(i, x) for i < g.MV receive the
+// results.  `phase` is the barrier's.  Every thread of the CTA calls it and
+// gets the status: 0, 1 for a zero divisor, 2 when the corrections or a wait
+// ran out.
+template <int P, typename LoadU, typename LoadV, typename StoreQ, typename StoreR>
+__device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P>& lay, uint8_t* smem, uint32_t tmem,
+                                             uint32_t& phase, LoadU load_u, LoadV load_v, StoreQ store_q,
+                                             StoreR store_r) {
+    using S = DtShape<P>;
+    constexpr int Q = S::Q, H = S::H, NT = S::NT, QT = S::QT;
+    const int tid = (int)threadIdx.x, lane = tid & 31;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    uint64_t* win = reinterpret_cast<uint64_t*>(smem + lay.win);
+    uint64_t* inv = reinterpret_cast<uint64_t*>(smem + lay.inv);
+    uint64_t* part = reinterpret_cast<uint64_t*>(smem + lay.part);
+    uint64_t* qraw = reinterpret_cast<uint64_t*>(smem + lay.qraw) + S::QLO;
+    uint64_t* qh = reinterpret_cast<uint64_t*>(smem + lay.qh);
+    int64_t* cs = reinterpret_cast<int64_t*>(smem + lay.cs);
+    uint32_t* scratch = reinterpret_cast<uint32_t*>(smem + lay.scratch);
+    const uint32_t sbase = tc_smem_addr(smem), bar = sbase + lay.bar;
+    const int MU = (int)g.MU, MV = (int)g.MV;
+
+    // ---- the divisor's size and shift
+    uint32_t top = 0;
+    for (int i = tid; i < MV; i += NT)
+        if (load_v((uint32_t)i) != 0) top = (uint32_t)i + 1;
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) scratch[warp] = top;
+    __syncthreads();
+    const int K = (int)__reduce_max_sync(0xffffffffu, lane < NT / 32 ? scratch[lane] : 0u);
+    __syncthreads();
+    if (K == 0) {
+        for (int i = tid; i < MU; i += NT) store_q((uint32_t)i, 0);
+        for (int i = tid; i < MV; i += NT) store_r((uint32_t)i, 0);
+        __syncthreads();
+        return 1;
+    }
+    const int s = __clzll((long long)load_v((uint32_t)K - 1));
+    const int Kp = K < 32 ? 32 : K, z = Kp - K;
+    // limb x of the divisor scaled by 2^s B^z, zero from Kp on
+    auto vlimb = [&](int x) -> uint64_t {
+        x -= z;
+        if (x < 0 || x >= K) return 0;
+        uint64_t v = load_v((uint32_t)x) << s;
+        if (s && x > 0) v |= load_v((uint32_t)x - 1) >> (64 - s);
+        return v;
+    };
+    const int nb = (MU + 1 - K + DT_KB - 1) / DT_KB;
+    const int len = nb * DT_KB + Kp;
+    const uint64_t vtop = vlimb(Kp - 1);
+
+    // ---- the reciprocal of the top 32 limbs, on one warp
+    if (warp == 0) {
+        qh[lane] = vlimb(Kp - 32 + lane);
+        if (lane < 2) qh[32 + lane] = 0;
+        inv[32 + lane] = 0;
+        __syncwarp();
+        dt_recip(qh, inv, part);
+    } else {
+        // the other warps: the window, the dividend scaled by 2^s B^z
+        for (int i = tid - 32; i < len; i += NT - 32) {
+            const int x = i - z;
+            uint64_t v = x >= 0 && x < MU ? load_u((uint32_t)x) << s : 0;
+            if (s && x > 0 && x <= MU) v |= load_u((uint32_t)x - 1) >> (64 - s);
+            win[S::at(i)] = v;
+        }
+        for (int i = tid - 32; i < S::R * Q; i += NT - 32) {
+            const int row = i / Q, q = i - row * Q, x = (row + S::KMIN) * Q + q;
+            if (x < 0 || x > Kp) *reinterpret_cast<uint4*>(smem + (q * S::R + row) * 16) = make_uint4(0, 0, 0, 0);
+        }
+        for (int i = tid - 32 - S::QLO; i < 32 + S::QHI; i += NT - 32)
+            if (i < 0 || i >= 32) qraw[i] = DT_HALF;
+    }
+    // ---- the divisor's balanced digits: Kp + 1 limbs of V + 0x8080..80
+    {
+        const int per = (Kp + 1 + NT - 1) / NT, lo = min(tid * per, Kp + 1), hi = min(lo + per, Kp + 1);
+        uint32_t c = 0, all = 1;
+        for (int x = lo; x < hi; x++) {
+            const uint64_t a = vlimb(x) + DT_HALF, t = a + c;
+            c = (a < DT_HALF) | (t < a);
+            all &= t == ~0ull;
+        }
+        c = block_carry_in(c, hi > lo ? (all & !c) : 1u, tid == 0, scratch);
+        for (int x = lo; x < hi; x++) {
+            const uint64_t a = vlimb(x) + DT_HALF, t = a + c;
+            c = (a < DT_HALF) | (t < a);
+            const uint32_t tl = (uint32_t)t, th = (uint32_t)(t >> 32);
+            const int row = x / Q - S::KMIN, q = x % Q;
+            *reinterpret_cast<uint4*>(smem + (q * S::R + row) * 16) =
+                make_uint4(dt_digits(tl, 0x4140), dt_digits(tl, 0x4342), dt_digits(th, 0x4140), dt_digits(th, 0x4342));
+        }
+    }
+    __syncthreads();
+
+    bool ok = true;
+    int fixes = 0;
+    for (int blk = nb - 1; blk >= 0; blk--) {
+        const int w0 = blk * DT_KB;          // the window: limbs w0 .. w0 + Kp + 30
+        // ---- estimate: columns 31 .. 62 of Wt inv, each warp its share of every column
+        {
+            uint64_t c0 = 0, c1 = 0;
+            uint32_t c2 = 0;
+            const uint64_t* iv = inv + 31 + lane - (int)warp;
+#pragma unroll
+            for (int e = 0; e < 1024 / NT; e++) mac3(c0, c1, c2, win[S::at(w0 + Kp - 1 + (int)warp + NT / 32 * e)], iv[-(NT / 32) * e]);
+            part[tid] = c0;
+            part[NT + tid] = c1;
+            part[2 * NT + tid] = c2;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            uint64_t lo = 0, mid = 0, hi = 0;
+#pragma unroll
+            for (int e = 0; e < NT / 32; e++) {
+                const uint64_t a = part[32 * e + lane], b = part[NT + 32 * e + lane];
+                lo += a;
+                const uint64_t cb = b + (lo < a);
+                mid += cb;
+                hi += part[2 * NT + 32 * e + lane] + (mid < cb) + (cb < b);
+            }
+            // limb i: the low part of column 32 + i, the middle of 31 + i, the high of 30 + i, and Wt
+            uint64_t x = __shfl_down_sync(0xffffffffu, lo, 1), y = __shfl_up_sync(0xffffffffu, hi, 1);
+            if (lane == 31) x = 0;
+            if (lane == 0) y = 0;
+            uint64_t sum = x + mid;
+            uint32_t e = sum < x;
+            sum += y;
+            e += sum < y;
+            const uint64_t wl = win[S::at(w0 + Kp - 1 + lane)];
+            sum += wl;
+            e += sum < wl;
+            uint32_t ein = __shfl_up_sync(0xffffffffu, e, 1), over;
+            if (lane == 0) ein = 0;
+            const uint64_t t = sum + ein;
+            const uint64_t fin = t + dt_lane_carry(t < ein, t == ~0ull, over);
+            over += __shfl_sync(0xffffffffu, e, 31);
+            uint64_t qt = __shfl_down_sync(0xffffffffu, fin, 1);
+            if (over) qt = ~0ull;
+            if (lane == 31) qt = 0;
+            qh[lane] = qt;
+            const uint64_t bt = qt + DT_HALF;
+            qraw[lane] = bt + dt_lane_carry(bt < DT_HALF, bt == ~0ull, over);
+        }
+        __syncthreads();
+        // ---- q^'s core matrices (multc.cuh's, of the balanced digits)
+        {
+            const uint32_t j1 = (tid & 7) + 1, sel = 0x3210u + 0x1111u * (j1 & 3);
+            const uint32_t* src = reinterpret_cast<const uint32_t*>(qraw) + 2 * (Q - 2 - S::T0 / 8 - (tid >> 3)) + (j1 >> 2);
+#pragma unroll
+            for (int e = 0; e < (S::CM + NT / 8 - 1) / (NT / 8); e++) {
+                if (NT / 8 * e + NT / 8 - 1 >= S::CM && NT / 8 * e + (tid >> 3) >= S::CM) break;
+                const uint32_t w0 = src[-NT / 4 * e], w1 = src[1 - NT / 4 * e], w2 = src[2 - NT / 4 * e];
+                const uint32_t zl = __byte_perm(w0, w1, sel), zh = __byte_perm(w1, w2, sel);
+                *reinterpret_cast<uint4*>(smem + lay.stage + tid * 16 + e * (NT * 16)) =
+                    make_uint4(dt_digits(zh, 0x4243), dt_digits(zh, 0x4041), dt_digits(zl, 0x4243), dt_digits(zl, 0x4041));
+            }
+        }
+        tc_fence_smem();
+        tc_fence_before();
+        __syncthreads();
+        if (warp == 0) {
+            tc_fence_after();
+            if (tc_elect()) {
+                const uint32_t da = tc_desc(sbase / 16, S::R), db = tc_desc((sbase + lay.stage) / 16, 8);
+#pragma unroll
+                for (int st = 0; st < S::STEPS; st++) {
+                    const int t = S::T0 + 16 * st, k = t >= 0 ? 0 : -((-t + P - 1) / P);
+                    tc_mma<P>(tmem, da + (uint32_t)((k - S::KMIN) + (t - k * P) / 8 * S::R), db + 16 * st, st > 0);
+                }
+                tc_commit(bar);
+            }
+            __syncwarp();
+        }
+        if (ok) ok = tc_warp_wait(bar, phase);
+        phase ^= 1;
+        tc_fence_after();
+        // ---- window -= q^ V.  Accumulator columns 8 n1 .. are limb Q - 1 - n1 of
+        // the row; with two threads a row the second four warps have its low
+        // half.  Segment sg is limbs QT sg ..; its carry out is signed, and made
+        // nonnegative for the next segment by 2^30, which that one has taken off.
+        const int half = H == 1 ? 0 : (int)(warp >> 2), sg = (tid & 127) * H + (H - 1 - half);
+        const int x0 = QT * sg, lim = Kp + DT_KB;
+        uint64_t d[QT];
+        int64_t c = sg == 0 ? 0 : -(1ll << 30);
+        const uint32_t tb = tmem + (((warp & 3) * 32) << 16) + half * (P / H);
+        auto limb_of = [&](int k, const float* v) {
+            int64_t u0 = 0, u1 = 0;
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                u0 += (int64_t)(int32_t)(__float_as_uint(v[e] + 12582912.0f) - 0x4B400000u) << (8 * e);
+                u1 += (int64_t)(int32_t)(__float_as_uint(v[4 + e] + 12582912.0f) - 0x4B400000u) << (8 * e);
+            }
+            const __int128 t = (__int128)(unsigned __int128)(x0 + k < lim ? win[S::at(w0 + x0 + k)] : 0) + c - u0 - ((__int128)u1 << 32);
+            d[k] = (uint64_t)t;
+            c = (int64_t)(t >> 64);
+        };
+#pragma unroll
+        for (int k = 0; k + 1 < QT; k += 2) {
+            float v[16];
+            tc_ld(tb + 8 * (QT - 2 - k), v);
+            limb_of(k, v + 8);
+            limb_of(k + 1, v);
+        }
+        if constexpr (QT % 2 == 1) {
+            float v[8];
+            tc_ld(tb, v);
+            limb_of(QT - 1, v);
+        }
+        cs[sg + 1] = c + (1ll << 30);
+        tc_fence_before();
+        __syncthreads();
+        const uint64_t in = sg == 0 ? 0 : (uint64_t)cs[sg];
+        uint64_t all = ~0ull;
+        uint32_t gen = 0;
+#pragma unroll
+        for (int k = 0; k < QT; k++) {
+            const uint64_t add = k == 0 ? in : gen;
+            d[k] += add;
+            gen = d[k] < add;
+            all &= d[k];
+        }
+        // carries between the segments, from every warp's masks
+        const bool prop = all == ~0ull && !gen;
+        {
+            const uint32_t G = __ballot_sync(0xffffffffu, gen != 0), Pm = __ballot_sync(0xffffffffu, prop);
+            if (lane == 0) {
+                scratch[2 * warp] = G;
+                scratch[2 * warp + 1] = Pm;
+            }
+        }
+        __syncthreads();
+        uint32_t cin = 0, crow = 0;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const uint32_t gu = scratch[2 * r], pu = scratch[2 * r + 1];
+            const uint32_t gl = H == 1 ? 0 : scratch[8 + 2 * r], pl = H == 1 ? ~0u : scratch[9 + 2 * r];
+            const uint32_t G = gu | (pu & gl);
+            const WarpCarry rc = warp_carry_resolve(G | (pu & pl), G, crow);
+            if (r == (int)(warp & 3)) {
+                const uint32_t low = rc.carries >> lane & 1u;
+                cin = H == 1 || half ? low : (gl >> lane & 1u) | ((pl >> lane & 1u) & low);
+            }
+            crow = rc.cout;
+        }
+        bool neg = sg == NT - 1 && c + (int64_t)(gen | (prop & cin)) < 0;
+#pragma unroll
+        for (int k = 0; k < QT; k++) {
+            const int x = x0 + k;
+            d[k] += cin;
+            cin = d[k] < cin;
+            if (x < lim) win[S::at(w0 + x)] = d[k];
+            // not below the divisor, perhaps
+            if ((x == Kp && d[k] != 0) || (x == Kp - 1 && d[k] >= vtop)) neg = true;
+        }
+        if (__syncthreads_or(neg)) {
+            // ---- correct: rare.  The limb above the window's Kp tells the sign.
+            const bool low = (win[S::at(w0 + Kp)] >> 63) != 0;
+            int step = 0;
+            __syncthreads();
+            for (int it = 0; it < DT_MAX_CORRECTIONS; it++) {
+                if (low) {
+                    step--;
+                    if (dt_addsub<S>(win, w0, [&](int i) { return vlimb(i); }, lim, false, scratch)) break;
+                } else {
+                    if (dt_addsub<S>(win, w0, [&](int i) { return vlimb(i); }, lim, true, scratch)) {
+                        dt_addsub<S>(win, w0, [&](int i) { return vlimb(i); }, lim, false, scratch);
+                        break;
+                    }
+                    step++;
+                }
+                if (it == DT_MAX_CORRECTIONS - 1) fixes = 1;
+            }
+            if (tid == 0 && step != 0) {          // the quotient block by as much
+                uint64_t k = (uint64_t)(step < 0 ? -step : step);
+                for (int i = 0; i < DT_KB && k; i++) {
+                    const uint64_t x = qh[i];
+                    qh[i] = step < 0 ? x - k : x + k;
+                    k = step < 0 ? x < k : qh[i] < k;
+                }
+            }
+            __syncthreads();
+        }
+        if (tid < DT_KB && blk * DT_KB + tid < MU) store_q((uint32_t)(blk * DT_KB + tid), qh[tid]);
+    }
+    // ---- the quotient's zero limbs, the remainder scaled back
+    for (int i = nb * DT_KB + tid; i < MU; i += NT) store_q((uint32_t)i, 0);
+    for (int i = tid; i < MV; i += NT) {
+        uint64_t x = 0;
+        if (i < K) {
+            x = win[S::at(z + i)] >> s;
+            if (s && i + 1 < K) x |= win[S::at(z + i + 1)] << (64 - s);
+        }
+        store_r((uint32_t)i, x);
+    }
+    return __syncthreads_or(!ok || fixes) ? 2 : 0;
+}
+
+}  // namespace bi

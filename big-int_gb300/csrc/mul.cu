@@ -402,20 +402,6 @@ mul_tc_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ 
         });
 }
 
-// CTAs an SM holds of a kernel that allocates tensor memory, from its
-// registers, shared memory and accumulator columns (the runtime's occupancy
-// query answers 1 for every such kernel).
-static int tc_ctas_per_sm(const void* kern, uint32_t threads, size_t smem, uint32_t cols) {
-    cudaFuncAttributes at;
-    if (cudaFuncGetAttributes(&at, kern) != cudaSuccess) {
-        cudaGetLastError();                    // not the launch's error
-        return 1;
-    }
-    const int by_regs = 65536 / (((at.numRegs + 7) / 8 * 8) * (int)threads);
-    const int by_smem = (int)(228 * 1024 / (smem + at.sharedSizeBytes + 1024)), by_cols = (int)(512 / cols);
-    return std::max(1, std::min(by_regs, std::min(by_smem, by_cols)));
-}
-
 template <typename T, int P>
 static bi_status mul_tc_launch(const T* a, const T* b, T* r, uint32_t m, uint64_t n, uint32_t L, uint32_t out_limbs,
                                uint32_t out_words, cudaStream_t st) {

@@ -193,8 +193,17 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// 16 or 32 accumulator columns of the warp's 32 rows; the wait is in the same
-// statement, so that no use of v can be scheduled before it
+// 8, 16 or 32 accumulator columns of the warp's 32 rows; the wait is in the
+// same statement, so that no use of v can be scheduled before it
+__device__ __forceinline__ void tc_ld(uint32_t addr, float (&v)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+        : "r"(addr)
+        : "memory");
+}
+
 __device__ __forceinline__ void tc_ld(uint32_t addr, float (&v)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
@@ -228,6 +237,37 @@ __device__ __forceinline__ uint32_t tc_digits(uint32_t w, uint32_t sel) {
     const uint32_t x = __byte_perm(w, 0x64646464u, sel);
     const __half2 y = __hsub2(*reinterpret_cast<const __half2*>(&x), __half2(__ushort_as_half(0x6400), __ushort_as_half(0x6400)));
     return *reinterpret_cast<const uint32_t*>(&y);
+}
+
+// COLS columns of tensor memory for the CTA, its address through the word at
+// shared address `at`; init() runs on one thread and its barriers are set up
+// for every thread and the tensor core when this returns.
+template <uint32_t COLS, typename Init>
+__device__ __forceinline__ uint32_t tc_alloc(uint32_t at, Init init) {
+    if (threadIdx.x == 0) {
+        init();
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at), "r"(COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    uint32_t tmem;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(at) : "memory");
+    return __shfl_sync(0xffffffffu, tmem, 0);
+}
+
+// Every thread, after the last use; the matrix instructions have ended.
+template <uint32_t COLS>
+__device__ __forceinline__ void tc_free(uint32_t tmem) {
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (threadIdx.x < 32)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -274,7 +314,11 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
     const uint32_t a_full = read + 8 * NS, a_empty = a_full + 16, done = a_empty + 16;
     static_assert(3 * NS + 4 + 2 <= 30, "barriers");
 
-    if (tid == 0) {
+    // the zero rows around a and the zero limbs around b stay zero
+    for (uint32_t idx = tid; idx < g.NA * ((lay.abytes + lay.bbytes) / 16); idx += S::THREADS)
+        *reinterpret_cast<uint4*>(smem + idx * 16) = make_uint4(0, 0, 0, 0);
+    tc_fence_smem();
+    const uint32_t tmem = tc_alloc<S::TMEM_COLS>(done + 8, [&] {
         for (uint32_t k = 0; k < NS; k++) {
             tc_bar_init(made + 8 * k, 1);
             tc_bar_init(run + 8 * k, 1);
@@ -285,21 +329,7 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
             tc_bar_init(a_empty + 8 * k, 6);
         }
         tc_bar_init(done, 2);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(done + 8), "r"(S::TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    // the zero rows around a and the zero limbs around b stay zero
-    for (uint32_t idx = tid; idx < g.NA * ((lay.abytes + lay.bbytes) / 16); idx += S::THREADS)
-        *reinterpret_cast<uint4*>(smem + idx * 16) = make_uint4(0, 0, 0, 0);
-    tc_fence_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(smem + (done + 8 - sbase)), 0);
+    });
 
     bool ok = true;
     uint32_t c = 0, p = 0;      // blocks and instances so far
@@ -476,11 +506,7 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
         }
     }
     if (!ok) atomicAdd(gave_up, 1u);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TMEM_COLS) : "memory");
+    tc_free<S::TMEM_COLS>(tmem);
 }
 
 }  // namespace bi

@@ -159,13 +159,14 @@ bi_status bi_div_u64(const uint64_t* u, const uint64_t* v, uint64_t* q, uint64_t
 bi_status bi_div_u32(const uint32_t* u, const uint32_t* v, uint32_t* q, uint32_t* r,
                      uint8_t* status, uint32_t mu, uint32_t mv, uint64_t n,
                      bi_stream stream);
-/* The method depends on the divisor's size in 64-bit limbs and on n (the */
-/* results do not: q and r are unique): schoolbook long division on one   */
-/* thread per instance up to 16 limbs and on one warp or lane group (8 or */
-/* 16 lanes, 1 to 32 limbs a lane) per instance up to 128 limbs, and up   */
-/* to 1024 limbs once n exceeds a few instances per SM (otherwise the     */
-/* shifted inverse on one CTA per instance); above 1024 limbs long        */
-/* division 8 quotient limbs at a time on two or four warps.              */
+/* The method depends on the sizes in 64-bit limbs and on n (the results do */
+/* not: q and r are unique): schoolbook long division on one thread per     */
+/* instance up to 16 divisor limbs and on one warp or lane group (8 or 16   */
+/* lanes, 1 to 32 limbs a lane) per instance up to 1024 limbs; long         */
+/* division 31 quotient limbs at a time on the tensor cores for divisors of */
+/* 40 (small batches) or 65 up to 2015 limbs once the quotient is long      */
+/* enough to earn back its setup; above that 8 quotient limbs at a time on  */
+/* four warps; the shifted inverse for few divisions with short quotients.  */
 /* The _shinv entries take the shifted inverse at every size (the         */
 /* reference's algorithm; dividends up to 2048 64-bit limbs, else         */
 /* BI_EUNSUPPORTED), the _long entries long division (divisors up to 4096 */
