@@ -20,8 +20,11 @@
 //     fastest in the batch), and the shifted
 //     inverse (divcore.cuh) on one 512-thread CTA per instance above -- and
 //     for a class above 128 limbs with too few divisions to fill the GPU,
-//     the crossover a uniform batch uses (div_use_long); most expensive
-//     first within a class.
+//     the crossover a uniform batch uses (div_use_long); divisors above 128
+//     limbs with quotients long enough to earn back the setup run 31 quotient
+//     limbs at a time on the tensor cores (divtc.cuh: the 20000-instance
+//     batch's divisions alone 1345 -> 216 us, the 100000-instance batch's 3292
+//     -> 928); most expensive first within a class.
 // The persistent kernels run concurrently on forked streams; the fork,
 // the launches, the counter reset and the join are captured once into a CUDA
 // graph and replayed by every bi_plan_execute.  Work is handed out with one
@@ -35,6 +38,7 @@
 #include "divblock.cuh"
 #include "divcore.cuh"
 #include "divsmall.cuh"
+#include "divtc.cuh"
 #include "mulcore.cuh"
 #include "mulwarp.cuh"
 #include "warpops.cuh"
@@ -210,13 +214,29 @@ constexpr int DIV_THREAD_CLASSES = 3, DIV_WARP_CLASSES = 8;
 constexpr uint32_t DIV_WARP_CLASS_MAX_MV[DIV_WARP_CLASSES] = {32, 64, 128, 256, 384, 512, 768, 1024};
 constexpr int DIV_CTA_CLASS = DIV_THREAD_CLASSES + DIV_WARP_CLASSES;
 constexpr int DIV_BLK2_CLASS = DIV_CTA_CLASS + 1, DIV_BLK4_CLASS = DIV_CTA_CLASS + 2;
-constexpr int DIV_CLASSES = DIV_CTA_CLASS + 3;
+// and long division in blocks on the tensor cores (divtc.cuh), by accumulator
+// width, for the divisions of batch_div_on_tc
+constexpr int DIV_TC_CLASSES = 5, DIV_TC0 = DIV_CTA_CLASS + 3;
+constexpr int DIV_TC_P[DIV_TC_CLASSES] = {16, 32, 64, 80, 128};
+constexpr int DIV_CLASSES = DIV_TC0 + DIV_TC_CLASSES;
 constexpr int DIV_CTA_THREADS = 512;
 // add/sub, multiply, one per division class, one per warp-multiply class
 constexpr int PLAN_KERNELS = 2 + DIV_CLASSES + MULW_CLASSES;
 constexpr int PLAN_MULW0 = 2 + DIV_CLASSES;      // index of the first warp-multiply kernel
 
-static inline int div_class(uint32_t mv) {
+// Divisions whose quotient is long enough to earn back the block division's
+// setup (div.cu's rule for a batch that fills the GPU; up to 128 limbs the
+// lane groups pack better beside the batch's other kernels).
+static inline bool batch_div_on_tc(uint32_t m, uint32_t mv) {
+    return mv > 128 && mv <= (uint32_t)DtShape<128>::MAX_K && (uint64_t)mv * (m - mv + 1) >= 9400;
+}
+
+static inline int div_class(uint32_t m, uint32_t mv) {
+    if (batch_div_on_tc(m, mv)) {
+        int c = 0;
+        while (mv > 16u * DIV_TC_P[c] - DT_KB - 2) c++;
+        return DIV_TC0 + c;
+    }
     if (mv <= 4) return 0;
     if (mv <= 8) return 1;
     if (mv <= 16) return 2;
@@ -389,6 +409,36 @@ batch_divblk_kernel(const bi_desc* __restrict__ descs, const uint32_t* __restric
     }
 }
 
+// Divisions in blocks on the tensor cores (divtc.cuh), one at a time a CTA;
+// `mu` sizes the window for the class's largest dividend.
+template <int P>
+__global__ void __launch_bounds__(DtShape<P>::NT)
+batch_divtc_kernel(const bi_desc* __restrict__ descs, const uint32_t* __restrict__ list, uint32_t count,
+                   uint32_t* counter, const uint64_t* in, uint64_t* out, uint8_t* flags, uint32_t mu) {
+    extern __shared__ __align__(128) uint8_t smem_dt[];
+    __shared__ uint32_t s_idx;
+    const DtSmem<P> lay(dt_geom(mu, 1, 8));
+    const uint32_t bar = tc_smem_addr(smem_dt) + lay.bar;
+    const uint32_t tmem = tc_alloc<DtShape<P>::TMEM_COLS>(bar + 8, [&] { tc_bar_init(bar, 1); });
+    uint32_t phase = 0;
+    for (;;) {
+        if (threadIdx.x == 0) s_idx = atomicAdd(counter, 1u);
+        __syncthreads();
+        const uint32_t idx = s_idx;
+        __syncthreads();
+        if (idx >= count) break;
+        const bi_desc d = descs[list[idx]];
+        const bool w32 = desc_w32(d);
+        auto lu = [&](uint32_t i) { return ld64(in, d.a, d.m, w32, i); };
+        auto lv = [&](uint32_t i) { return ld64(in, d.b, d.mb, w32, i); };
+        auto sq = [&](uint32_t i, uint64_t x) { st64(out, d.r, d.m, w32, i, x); };
+        auto sr = [&](uint32_t i, uint64_t x) { st64(out, d.r2, d.mb, w32, i, x); };
+        const uint8_t st = dt_divide<P>(dt_geom(m64(d), mb64(d), 8), lay, smem_dt, tmem, phase, lu, lv, sq, sr);
+        if (flags && threadIdx.x == 0) flags[d.flag] = st;
+    }
+    tc_free<DtShape<P>::TMEM_COLS>(tmem);
+}
+
 struct bi_plan {
     int device = 0;
     uint64_t count = 0;
@@ -403,6 +453,7 @@ struct bi_plan {
     uint32_t n_addsub = 0, n_mul = 0, n_items = 0, n_div = 0, n_items_large = 0, n_mulw_total = 0;
     uint32_t mulw_off[MULW_CLASSES] = {}, n_mulw[MULW_CLASSES] = {};
     uint32_t div_off[DIV_CLASSES] = {}, n_divc[DIV_CLASSES] = {};
+    uint32_t divc_mu[DIV_TC_CLASSES] = {};   // largest dividend of each tensor-core class (its shared window)
     uint32_t max_mul_Lp_full = 0, max_mul_Lp_trunc = 0;
     uint64_t nflags = 0;                // flag-arena bytes the descriptors were checked against
     size_t mul_smem = 0, div_smem = 0, divc_smem[DIV_CLASSES] = {};
@@ -453,7 +504,7 @@ static void div_class_map(const bi_desc* descs, const uint32_t* div, uint32_t n,
     uint64_t cnt[DIV_CLASSES] = {};
     uint32_t max_m[DIV_CLASSES] = {};
     for (uint32_t k = 0; k < n; k++) {
-        const int c = div_class(mb64(descs[div[k]]));
+        const int c = div_class(m64(descs[div[k]]), mb64(descs[div[k]]));
         cnt[c]++;
         max_m[c] = std::max(max_m[c], m64(descs[div[k]]));
     }
@@ -477,14 +528,26 @@ static void div_class_map(const bi_desc* descs, const uint32_t* div, uint32_t n,
 
 // Division order: by class, then most expensive first.
 static bool div_before(const bi_desc& x, const bi_desc& y, const int* map) {
-    const int cx = map[div_class(mb64(x))], cy = map[div_class(mb64(y))];
+    const int cx = map[div_class(m64(x), mb64(x))], cy = map[div_class(m64(y), mb64(y))];
     if (cx != cy) return cx < cy;
     return (uint64_t)m64(x) * mb64(x) > (uint64_t)m64(y) * mb64(y);
 }
 
 // Per-class offsets, counts and shared memory of a division list sorted by div_before.
+static size_t div_tc_smem(int k, uint32_t mu) {
+    const DtGeom g = dt_geom(mu, 1, 8);
+    switch (k) {
+    case 0: return DtSmem<16>(g).total;
+    case 1: return DtSmem<32>(g).total;
+    case 2: return DtSmem<64>(g).total;
+    case 3: return DtSmem<80>(g).total;
+    default: return DtSmem<128>(g).total;
+    }
+}
+
 static void div_classes(bi_plan* p, const bi_desc* descs, const uint32_t* div, uint32_t n, const int* map) {
     p->div_smem = 0;
+    for (uint32_t& mu : p->divc_mu) mu = 0;
     for (int c = 0; c < DIV_CLASSES; c++) {
         p->div_off[c] = 0;
         p->n_divc[c] = 0;
@@ -492,9 +555,13 @@ static void div_classes(bi_plan* p, const bi_desc* descs, const uint32_t* div, u
     }
     for (uint32_t k = 0; k < n; k++) {
         const bi_desc& d = descs[div[k]];
-        const int c = map[div_class(mb64(d))];
+        const int c = map[div_class(m64(d), mb64(d))];
         if (p->n_divc[c]++ == 0) p->div_off[c] = k;
         if (c == DIV_CTA_CLASS) p->divc_smem[c] = std::max(p->divc_smem[c], div_smem_bytes(div_geom(m64(d), mb64(d), 8)));
+        if (c >= DIV_TC0) {
+            p->divc_mu[c - DIV_TC0] = std::max(p->divc_mu[c - DIV_TC0], m64(d));
+            p->divc_smem[c] = div_tc_smem(c - DIV_TC0, p->divc_mu[c - DIV_TC0]);
+        }
         p->div_smem = std::max(p->div_smem, p->divc_smem[c]);
     }
 }
@@ -518,8 +585,14 @@ static bi_status grid_for(const void* k, int threads, size_t smem, uint64_t work
 // The kernel of division class c (host-side function pointer) and its CTA width.
 static const void* div_class_kernel(int c, int* threads) {
     *threads = c < DIV_THREAD_CLASSES ? DIV_THREAD_CTA : c < DIV_CTA_CLASS ? DIV_WARP_CTA
-               : c == DIV_BLK2_CLASS ? 64 : c == DIV_BLK4_CLASS ? 128 : DIV_CTA_THREADS;
+               : c == DIV_BLK2_CLASS ? 64 : c == DIV_BLK4_CLASS ? 128
+               : c < DIV_TC0 ? DIV_CTA_THREADS : DIV_TC_P[c - DIV_TC0] >= 80 ? 256 : 128;
     switch (c) {
+    case DIV_TC0: return (const void*)batch_divtc_kernel<16>;
+    case DIV_TC0 + 1: return (const void*)batch_divtc_kernel<32>;
+    case DIV_TC0 + 2: return (const void*)batch_divtc_kernel<64>;
+    case DIV_TC0 + 3: return (const void*)batch_divtc_kernel<80>;
+    case DIV_TC0 + 4: return (const void*)batch_divtc_kernel<128>;
     case DIV_BLK2_CLASS: return (const void*)batch_divblk_kernel<2>;
     case DIV_BLK4_CLASS: return (const void*)batch_divblk_kernel<4>;
     case 0: return (const void*)batch_divthread_kernel<4>;
@@ -594,6 +667,14 @@ static bi_status prepare_launch(bi_plan* p, const BatchTune& t, Launch3* L) {
         const void* k = div_class_kernel(c, &threads);
         // instances per CTA: one a thread, one a lane group (8, 16 or 32 lanes), one a CTA
         static constexpr uint32_t group_ipw[DIV_WARP_CLASSES] = {4, 4, 2, 1, 2, 1, 1, 1};
+        if (c >= DIV_TC0) {
+            if (smem_opt_in(k, L->smem[2 + c]) != cudaSuccess)
+                return set_error(BI_ECUDA, "batch kernel setup: %s", cudaGetErrorString(cudaGetLastError()));
+            const int cols = (int)tc_pow2((uint32_t)DIV_TC_P[c - DIV_TC0]);
+            L->grid[2 + c] = (unsigned)std::min<uint64_t>(
+                n, (uint64_t)sms * tc_ctas_per_sm(k, (uint32_t)threads, L->smem[2 + c], (uint32_t)cols));
+            continue;
+        }
         const uint64_t per = c < DIV_THREAD_CLASSES ? (uint64_t)threads
                              : c < DIV_CTA_CLASS    ? (uint64_t)threads / 32 * group_ipw[c - DIV_THREAD_CLASSES]
                                                     : 1;
@@ -667,6 +748,11 @@ static bi_status launch_plan_kernels(bi_plan* p, const uint64_t* in, uint64_t* o
             case 8: batch_divwarp_kernel<16><<<grid, DIV_WARP_CTA, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             case 9: batch_divwarp3_kernel<24><<<grid, DIV_WARP_CTA, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             case 10: batch_divwarp_kernel<32><<<grid, DIV_WARP_CTA, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
+            case DIV_TC0: batch_divtc_kernel<16><<<grid, DtShape<16>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[0]); break;
+            case DIV_TC0 + 1: batch_divtc_kernel<32><<<grid, DtShape<32>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[1]); break;
+            case DIV_TC0 + 2: batch_divtc_kernel<64><<<grid, DtShape<64>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[2]); break;
+            case DIV_TC0 + 3: batch_divtc_kernel<80><<<grid, DtShape<80>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[3]); break;
+            case DIV_TC0 + 4: batch_divtc_kernel<128><<<grid, DtShape<128>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[4]); break;
             case DIV_BLK2_CLASS: batch_divblk_kernel<2><<<grid, 64, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             case DIV_BLK4_CLASS: batch_divblk_kernel<4><<<grid, 128, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             default:
