@@ -11,7 +11,12 @@
 //     futhark/sub.fut:14-16) -- no shared memory and no CTA barrier, so any
 //     size mix keeps the warps busy;
 //   * multiplications are bucketed by padded size; a persistent CTA takes a
-//     bucket item (as many instances as fit one CTA, mulcore.cuh);
+//     bucket item (as many instances as fit one CTA, mulcore.cuh); full
+//     products of 160 limbs or more and truncated ones of 208 or more go to
+//     persistent tensor-core kernels by accumulator width (multc.cuh; the
+//     20000-instance batch's multiplies alone 590 -> 219 us, the 100000's 2817
+//     -> 965; the kernel's 512 threads fill an SM's registers, so they run
+//     beside the divisions only from SM to SM);
 //   * divisions go to persistent kernels by divisor size class: schoolbook
 //     long division (divsmall.cuh) on one thread per instance for divisors
 //     up to 4, 8 and 16 limbs, on one lane group per instance up to 32, 64,
@@ -40,6 +45,7 @@
 #include "divsmall.cuh"
 #include "divtc.cuh"
 #include "mulcore.cuh"
+#include "multc.cuh"
 #include "mulwarp.cuh"
 #include "warpops.cuh"
 
@@ -221,8 +227,10 @@ constexpr int DIV_TC_P[DIV_TC_CLASSES] = {16, 32, 64, 80, 128};
 constexpr int DIV_CLASSES = DIV_TC0 + DIV_TC_CLASSES;
 constexpr int DIV_CTA_THREADS = 512;
 // add/sub, multiply, one per division class, one per warp-multiply class
-constexpr int PLAN_KERNELS = 2 + DIV_CLASSES + MULW_CLASSES;
+constexpr int MUL_TC_CLASSES = 3;
+constexpr int PLAN_KERNELS = 2 + DIV_CLASSES + MULW_CLASSES + MUL_TC_CLASSES;
 constexpr int PLAN_MULW0 = 2 + DIV_CLASSES;      // index of the first warp-multiply kernel
+constexpr int PLAN_MULTC0 = PLAN_MULW0 + MULW_CLASSES;   // and of the first tensor-core multiply kernel
 
 // Divisions whose quotient is long enough to earn back the block division's
 // setup (div.cu's rule for a batch that fills the GPU; up to 128 limbs the
@@ -244,6 +252,43 @@ static inline int div_class(uint32_t m, uint32_t mv) {
     int c = 0;
     while (DIV_WARP_CLASS_MAX_MV[c] < mv) c++;
     return DIV_THREAD_CLASSES + c;
+}
+
+// Multiplies on the tensor cores (multc.cuh) by the accumulator width that
+// holds the product: up to 512, 1024 and more product limbs.  The sizes are
+// the uniform entry's for batches that fill the GPU.
+constexpr int MUL_TC_P[MUL_TC_CLASSES] = {32, 64, 128};
+constexpr uint32_t BATCH_TC_FULL_L = 160, BATCH_TC_TRUNC_L = 208;
+inline int multc_class(uint32_t m, bool full) {
+    if (m < (full ? BATCH_TC_FULL_L : BATCH_TC_TRUNC_L)) return -1;
+    const uint32_t out = full ? 2 * m : m;
+    return out <= 16 * 32 ? 0 : out <= 16 * 64 ? 1 : 2;
+}
+
+struct TcItem {                        // an instance of the batch
+    const uint64_t* in;
+    uint64_t* out;
+    uint64_t oa, ob, orr;
+    uint32_t m, outm, L, out_limbs;
+    bool w32;
+    __device__ __forceinline__ uint64_t a(uint32_t x) const { return ld64(in, oa, m, w32, x); }
+    __device__ __forceinline__ uint64_t b(uint32_t x) const { return ld64(in, ob, m, w32, x); }
+    __device__ __forceinline__ void store(uint32_t x, uint64_t v) const { st64(out, orr, outm, w32, x, v); }
+};
+
+__device__ uint32_t batch_tc_gave_up;    // waits on the tensor core that ran out (never seen)
+
+template <int P>
+__global__ void __launch_bounds__(TcShape<P>::THREADS, 1)
+batch_multc_kernel(const bi_desc* __restrict__ descs, const uint32_t* __restrict__ list, uint32_t count,
+                   const uint64_t* in, uint64_t* out, TcGeom g) {
+    extern __shared__ __align__(128) uint8_t smem_tc[];
+    tc_products<P>(g, smem_tc, blockIdx.x, gridDim.x, count, &batch_tc_gave_up, [&](uint64_t i) {
+        const bi_desc& d = descs[list[i]];
+        const uint32_t m = d.m, outm = d.op == BI_OP_MULFULL ? 2 * m : m;
+        const bool w32 = desc_w32(d);
+        return TcItem{in, out, d.a, d.b, d.r, m, outm, w32 ? (m + 1) / 2 : m, w32 ? (outm + 1) / 2 : outm, w32};
+    });
 }
 
 template <int MX>
@@ -448,6 +493,9 @@ struct bi_plan {
     uint32_t* d_div = nullptr;          // division list: class 0, then 1, then 2
     MulItem* d_items = nullptr;         // every multiply, on the CTA kernel
     MulItem* d_items_large = nullptr;   // the multiplies the warp classes do not take
+    uint32_t* d_multc = nullptr;        // large products: tensor-core class 0, then 1, then 2
+    uint32_t multc_off[MUL_TC_CLASSES] = {}, n_multc[MUL_TC_CLASSES] = {};
+    TcGeom multc_geom[MUL_TC_CLASSES] = {};
     uint32_t* d_mulw = nullptr;         // small full products: warp class 0, then 1, ...
     uint32_t* d_counters = nullptr;     // one per kernel (PLAN_KERNELS)
     uint32_t n_addsub = 0, n_mul = 0, n_items = 0, n_div = 0, n_items_large = 0, n_mulw_total = 0;
@@ -626,6 +674,21 @@ static const void* mulw_class_kernel(int c) {
     }
 }
 
+// The tensor-core multiply kernel of class c, its threads, accumulator
+// columns and shared memory.
+template <int C>
+static const void* multc_kernel(const TcGeom& g, uint32_t* threads, uint32_t* cols, size_t* smem) {
+    constexpr int P = MUL_TC_P[C];
+    *threads = TcShape<P>::THREADS;
+    *cols = TcShape<P>::TMEM_COLS;
+    *smem = TcSmem<P>(g).total;
+    return (const void*)batch_multc_kernel<P>;
+}
+static const void* multc_class_kernel(int c, const TcGeom& g, uint32_t* threads, uint32_t* cols, size_t* smem) {
+    return c == 0 ? multc_kernel<0>(g, threads, cols, smem) : c == 1 ? multc_kernel<1>(g, threads, cols, smem)
+                                                                    : multc_kernel<2>(g, threads, cols, smem);
+}
+
 // Grid sizes and shared memory of the kernels for tuning t; sets the
 // kernels' shared-memory limits (done outside any stream capture).
 static bi_status prepare_launch(bi_plan* p, const BatchTune& t, Launch3* L) {
@@ -642,6 +705,17 @@ static bi_status prepare_launch(bi_plan* p, const BatchTune& t, Launch3* L) {
     for (int c = 0; c < MULW_CLASSES; c++) {
         L->smem[PLAN_MULW0 + c] = 0;
         L->grid[PLAN_MULW0 + c] = 0;
+    }
+    for (int c = 0; c < MUL_TC_CLASSES; c++) {
+        L->smem[PLAN_MULTC0 + c] = 0;
+        L->grid[PLAN_MULTC0 + c] = 0;
+        if (!p->n_multc[c]) continue;
+        uint32_t threads = 0, cols = 0;
+        const void* k = multc_class_kernel(c, p->multc_geom[c], &threads, &cols, &L->smem[PLAN_MULTC0 + c]);
+        if (smem_opt_in(k, L->smem[PLAN_MULTC0 + c]) != cudaSuccess)
+            return set_error(BI_ECUDA, "batch kernel setup: %s", cudaGetErrorString(cudaGetLastError()));
+        L->grid[PLAN_MULTC0 + c] = (unsigned)std::min<uint64_t>(
+            p->n_multc[c], (uint64_t)sms * tc_ctas_per_sm(k, threads, L->smem[PLAN_MULTC0 + c], cols));
     }
     int occ = 1;
     L->grid[1] = 0;
@@ -725,6 +799,16 @@ static bi_status launch_plan_kernels(bi_plan* p, const uint64_t* in, uint64_t* o
             default: batch_mulwarp_kernel<32><<<grid, MUL_WARP_CTA, smem, st>>>(p->d_descs, list, n, ctr, in, out);
             }
             BI_RETURN_IF(check_launch("batch warp mul kernel"));
+        }
+        for (int c = MUL_TC_CLASSES - 1; c >= 0; c--) {
+            uint32_t n = p->n_multc[c], threads = 0, cols = 0;
+            if (!n) continue;
+            size_t smem = 0;
+            const void* k = multc_class_kernel(c, p->multc_geom[c], &threads, &cols, &smem);
+            const uint32_t* list = p->d_multc + p->multc_off[c];
+            void* args[] = {&p->d_descs, &list, &n, &in, &out, &p->multc_geom[c]};
+            cudaLaunchKernel(k, dim3(L.grid[PLAN_MULTC0 + c]), dim3(threads), args, smem, s[PLAN_MULTC0 + c]);
+            BI_RETURN_IF(check_launch("batch tensor mul kernel"));
         }
     }
     if (comps & COMP_DIV) {
@@ -814,6 +898,7 @@ static void plan_free(bi_plan* p) {
     cudaFree(p->d_items);
     cudaFree(p->d_items_large);
     cudaFree(p->d_mulw);
+    cudaFree(p->d_multc);
     cudaFree(p->d_counters);
     for (int k = 0; k < PLAN_KERNELS; k++) {
         if (p->side[k]) cudaStreamDestroy(p->side[k]);
@@ -890,7 +975,7 @@ bi_status bi_plan_create(bi_plan** out_plan, const bi_desc* descs, uint64_t coun
     cudaGetDevice(&p->device);
     p->count = count;
     p->nflags = nflags;
-    std::vector<uint32_t> addsub, div, mulw[MULW_CLASSES];
+    std::vector<uint32_t> addsub, div, mulw[MULW_CLASSES], multc[MUL_TC_CLASSES];
     std::vector<std::pair<uint64_t, uint32_t>> mulkeys;   // (bucket key, index)
     for (uint64_t i = 0; i < count; i++) {
         const bi_desc& d = descs[i];
@@ -903,6 +988,11 @@ bi_status bi_plan_create(bi_plan** out_plan, const bi_desc* descs, uint64_t coun
         case BI_OP_MULFULL: {
             const uint32_t Lp = (m64(d) + 2 * MUL_C - 1) / (2 * MUL_C) * (2 * MUL_C);
             const uint32_t full = d.op == BI_OP_MULFULL;
+            const int tc = multc_class(m64(d), full != 0);
+            if (tc >= 0) {
+                multc[tc].push_back((uint32_t)i);
+                break;
+            }
             if (full) p->max_mul_Lp_full = std::max(p->max_mul_Lp_full, Lp);
             else p->max_mul_Lp_trunc = std::max(p->max_mul_Lp_trunc, Lp);
             mulkeys.push_back({((uint64_t)full << 40) | ((uint64_t)Lp << 8), (uint32_t)i});
@@ -952,9 +1042,31 @@ bi_status bi_plan_create(bi_plan** out_plan, const bi_desc* descs, uint64_t coun
         mulw_all.insert(mulw_all.end(), mulw[c].begin(), mulw[c].end());
     }
     p->n_mulw_total = (uint32_t)mulw_all.size();
+    // the tensor-core classes: a CTA takes every grid-th instance, most work first
+    std::vector<uint32_t> multc_all;
+    for (int c = 0; c < MUL_TC_CLASSES; c++) {
+        auto cost = [&](uint32_t x) { return (uint64_t)m64(descs[x]) * (descs[x].op == BI_OP_MULFULL ? 2 : 1); };
+        std::stable_sort(multc[c].begin(), multc[c].end(), [&](uint32_t x, uint32_t y) { return cost(x) > cost(y); });
+        p->multc_off[c] = (uint32_t)multc_all.size();
+        p->n_multc[c] = (uint32_t)multc[c].size();
+        TcGeom g = {};
+        for (uint32_t x : multc[c]) {
+            const uint32_t L = m64(descs[x]), out = descs[x].op == BI_OP_MULFULL ? 2 * L : L;
+            if (c == 0) tc_geometry_add<MUL_TC_P[0]>(g, L, out);
+            else if (c == 1) tc_geometry_add<MUL_TC_P[1]>(g, L, out);
+            else tc_geometry_add<MUL_TC_P[2]>(g, L, out);
+        }
+        g.NA = 2;
+        uint32_t threads, cols;
+        size_t smem;
+        multc_class_kernel(c, g, &threads, &cols, &smem);
+        if (smem > 227 * 1024) g.NA = 1;
+        p->multc_geom[c] = g;
+        multc_all.insert(multc_all.end(), multc[c].begin(), multc[c].end());
+    }
     p->n_items_large = (uint32_t)items_large.size();
     p->n_addsub = (uint32_t)addsub.size();
-    p->n_mul = (uint32_t)mul.size();
+    p->n_mul = (uint32_t)(mul.size() + multc_all.size());
     p->n_items = (uint32_t)items.size();
     p->n_div = (uint32_t)div.size();
     div_classes(p, descs, div.data(), p->n_div, dmap);
@@ -978,6 +1090,7 @@ bi_status bi_plan_create(bi_plan** out_plan, const bi_desc* descs, uint64_t coun
     if (st == BI_OK) st = dev_upload(&p->d_items, items, p->cap);
     if (st == BI_OK) st = dev_upload(&p->d_items_large, items_large, p->cap);
     if (st == BI_OK) st = dev_upload(&p->d_mulw, mulw_all, p->cap);
+    if (st == BI_OK) st = dev_upload(&p->d_multc, multc_all, p->cap);
     if (st == BI_OK) {
         std::vector<uint32_t> zeros(PLAN_KERNELS, 0);
         st = dev_upload(&p->d_counters, zeros, p->cap);

@@ -378,36 +378,42 @@ static bi_status mul_thread(const T* a, const T* b, T* r, uint32_t m, uint64_t n
 // ---------------------------------------------------------------------------
 __device__ uint32_t tc_gave_up;    // waits on the tensor core that ran out (never seen)
 
+template <typename T>
+struct TcRow {                         // an instance of a uniform batch
+    const T *pa, *pb;
+    T* pr;
+    uint32_t m, L, out_words, out_limbs;
+    static __device__ __forceinline__ uint64_t limb(const T* row, uint32_t m, uint32_t x) {
+        if constexpr (sizeof(T) == 8) return row[x];
+        else return row[2 * x] | (2 * x + 1 < m ? (uint64_t)row[2 * x + 1] << 32 : 0ull);
+    }
+    __device__ __forceinline__ uint64_t a(uint32_t x) const { return limb(pa, m, x); }
+    __device__ __forceinline__ uint64_t b(uint32_t x) const { return limb(pb, m, x); }
+    __device__ __forceinline__ void store(uint32_t x, uint64_t v) const {
+        if constexpr (sizeof(T) == 8) {
+            pr[x] = v;
+        } else {                          // an odd m leaves the top limbs without words
+            if (2 * x < out_words) pr[2 * x] = (uint32_t)v;
+            if (2 * x + 1 < out_words) pr[2 * x + 1] = (uint32_t)(v >> 32);
+        }
+    }
+};
+
 template <typename T, int P>
 __global__ void __launch_bounds__(TcShape<P>::THREADS, 1)
-mul_tc_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ r, uint64_t n, TcGeom g) {
+mul_tc_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ r, uint64_t n, TcGeom g, uint32_t m,
+              uint32_t out_words, uint32_t out_limbs) {
     extern __shared__ __align__(128) uint8_t smem_tc[];
-    auto limb = [&](const T* p, uint64_t inst, uint32_t x) -> uint64_t {
-        const T* row = p + inst * g.m;
-        if constexpr (sizeof(T) == 8) return row[x];
-        else return row[2 * x] | (2 * x + 1 < g.m ? (uint64_t)row[2 * x + 1] << 32 : 0ull);
-    };
-    tc_products<P>(
-        g, smem_tc, blockIdx.x, gridDim.x, n, &tc_gave_up,
-        [&](uint64_t inst, uint32_t x) { return limb(a, inst, x); },
-        [&](uint64_t inst, uint32_t x) { return limb(b, inst, x); },
-        [&](uint64_t inst, uint32_t x, uint64_t v) {
-            T* row = r + inst * g.out_words;
-            if constexpr (sizeof(T) == 8) {
-                row[x] = v;
-            } else {                          // an odd m leaves the top limbs without words
-                if (2 * x < g.out_words) row[2 * x] = (uint32_t)v;
-                if (2 * x + 1 < g.out_words) row[2 * x + 1] = (uint32_t)(v >> 32);
-            }
-        });
+    tc_products<P>(g, smem_tc, blockIdx.x, gridDim.x, n, &tc_gave_up, [&](uint64_t inst) {
+        return TcRow<T>{a + inst * m, b + inst * m, r + inst * out_words, m, g.L, out_words, out_limbs};
+    });
 }
 
 template <typename T, int P>
 static bi_status mul_tc_launch(const T* a, const T* b, T* r, uint32_t m, uint64_t n, uint32_t L, uint32_t out_limbs,
                                uint32_t out_words, cudaStream_t st) {
-    TcGeom g = tc_geometry<P>(L, out_limbs);
-    g.m = m;
-    g.out_words = out_words;
+    TcGeom g = {};
+    tc_geometry_add<P>(g, L, out_limbs);
     g.NA = 2;
     if (TcSmem<P>(g).total > 227 * 1024) g.NA = 1;
     const size_t smem = TcSmem<P>(g).total;
@@ -415,7 +421,7 @@ static bi_status mul_tc_launch(const T* a, const T* b, T* r, uint32_t m, uint64_
     cudaError_t e = smem_opt_in((const void*)kern, smem);
     if (e != cudaSuccess) return set_error(BI_ECUDA, "mul: %s", cudaGetErrorString(e));
     const uint64_t cap = (uint64_t)num_sms() * tc_ctas_per_sm((const void*)kern, TcShape<P>::THREADS, smem, TcShape<P>::TMEM_COLS);
-    kern<<<(unsigned)(n < cap ? n : cap), TcShape<P>::THREADS, smem, st>>>(a, b, r, n, g);
+    kern<<<(unsigned)(n < cap ? n : cap), TcShape<P>::THREADS, smem, st>>>(a, b, r, n, g, m, out_words, out_limbs);
     return check_launch("mul tensor kernel");
 }
 

@@ -52,47 +52,46 @@ struct TcShape {
     static constexpr uint32_t THREADS = DRAIN + 256;
 };
 
+// The layout of a kernel's operand buffers, for every instance it is given.
 struct TcGeom {
-    uint32_t L;            // limbs per operand in the u64 view
-    uint32_t m;            // limbs per operand in the caller's type
-    uint32_t out_limbs;    // result limbs in the u64 view
-    uint32_t out_words;    // result limbs in the caller's type
-    uint32_t D;            // rows of P digits that hold a
+    uint32_t L;            // limbs of the largest operand, in the u64 view
     uint32_t R;            // rows of the A buffer (R % 8 == 1: consecutive limbs fall into different banks)
     int32_t rho0;          // a's row at the buffer's first row (<= 0: zero rows before a)
-    uint32_t tiles;        // accumulator tiles of 128 rows
     uint32_t NA;           // operand buffers (2: the next instance is loaded under this one's product)
 };
 
 // first and last row offset k of tile tau (t = P k ..): rows 128 tau + i + k
-// that meet a, terms that meet b
+// that meet a's D rows, terms that meet b
 __host__ __device__ inline void tc_krange(uint32_t D, uint32_t tau, int& lo, int& hi) {
     const int a = -(int)(128 * tau + 127), b = (int)D - 1 - (int)(128 * tau);
     lo = a > -(int)D ? a : -(int)D;
     hi = b < 0 ? b : 0;
 }
 
+// rows of P digits that hold L limbs, accumulator tiles of 128 rows that hold out_limbs
 template <int P>
-__host__ __device__ inline TcGeom tc_geometry(uint32_t L, uint32_t out_limbs) {
+__host__ __device__ inline uint32_t tc_rows(uint32_t L) { return (L + P / 8 - 1) / (P / 8); }
+template <int P>
+__host__ __device__ inline uint32_t tc_tiles(uint32_t out_limbs) { return (out_limbs + 16 * P - 1) / (16 * P); }
+
+// Widens g (zero at first) for products of L limbs to out_limbs.
+template <int P>
+inline void tc_geometry_add(TcGeom& g, uint32_t L, uint32_t out_limbs) {
     using S = TcShape<P>;
-    TcGeom g;
-    g.L = g.m = L;
-    g.out_limbs = g.out_words = out_limbs;
-    g.D = (L + S::Q - 1) / S::Q;
-    g.tiles = (out_limbs + 128 * S::Q - 1) / (128 * S::Q);
-    int first = 0, last = 0;
-    for (uint32_t tau = 0; tau < g.tiles; tau++) {
+    int first = g.rho0, last = g.L ? g.rho0 + (int)g.R - 1 : first;
+    const uint32_t D = tc_rows<P>(L);
+    for (uint32_t tau = 0; tau < tc_tiles<P>(out_limbs); tau++) {
         int lo, hi;
-        tc_krange(g.D, tau, lo, hi);
+        tc_krange(D, tau, lo, hi);
         const int nblk = (hi - lo + S::RB) / S::RB;
         const int f = (int)(128 * tau) + lo, l = (int)(128 * tau) + 127 + lo + nblk * S::RB - 1;
-        if (tau == 0 || f < first) first = f;
-        if (tau == 0 || l > last) last = l;
+        first = f < first ? f : first;
+        last = l > last ? l : last;
     }
+    if (L > g.L) g.L = L;
     g.rho0 = first;
     g.R = (uint32_t)(last - first + 1);
     g.R += (9 - g.R % 8) % 8;
-    return g;
 }
 
 // Shared memory in bytes: NA times A, NA times b's limbs, the stages of B, the
@@ -279,9 +278,10 @@ __device__ __forceinline__ void tc_free(uint32_t tmem) {
 //   issuing   the matrix instructions, into NS accumulators in turn;
 //   draining  each finished accumulator into 32-bit sums, then the product's
 //             limbs, while the tensor core is on the next blocks or instance.
-// load_a(i, x), load_b(i, x) give limb x < g.L of instance i's operands,
-// store(i, x, v) receives limb x < g.out_limbs of its product mod B^out_limbs.
-// Every wait gives up after a second; the CTA then leaves and the call is
+// fetch(i) gives instance i: L (at most g.L) and out_limbs, a(x) and b(x) the
+// limbs of its operands (x < L), store(x, v) takes limb x < out_limbs of its
+// product mod B^out_limbs.  Each role fetches an instance while it works on
+// the one before.  Every wait gives up after a second; the CTA then leaves and the call is
 // counted in `gave_up`.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t tc_carry_in(uint32_t g, uint32_t p, uint32_t nwarps, uint32_t* scratch) {
@@ -298,9 +298,9 @@ __device__ __forceinline__ uint32_t tc_carry_in(uint32_t g, uint32_t p, uint32_t
     return (warp_carry_resolve(A, B, cin).carries >> lane) & 1u;
 }
 
-template <int P, typename LoadA, typename LoadB, typename Store>
+template <int P, typename Fetch>
 __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint64_t first, uint64_t step, uint64_t n,
-                                            uint32_t* gave_up, LoadA load_a, LoadB load_b, Store store) {
+                                            uint32_t* gave_up, Fetch fetch) {
     using S = TcShape<P>;
     constexpr int Q = S::Q, QT = S::QT, CT = S::CT;
     constexpr uint32_t ND = S::DRAIN, NS = S::NS;
@@ -314,7 +314,7 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
     const uint32_t a_full = read + 8 * NS, a_empty = a_full + 16, done = a_empty + 16;
     static_assert(3 * NS + 4 + 2 <= 30, "barriers");
 
-    // the zero rows around a and the zero limbs around b stay zero
+    // rows around a and limbs around b are zero, and stay so
     for (uint32_t idx = tid; idx < g.NA * ((lay.abytes + lay.bbytes) / 16); idx += S::THREADS)
         *reinterpret_cast<uint4*>(smem + idx * 16) = make_uint4(0, 0, 0, 0);
     tc_fence_smem();
@@ -336,21 +336,31 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
     if (warp >= ND / 32 + 6) {
         // ---- loading
         const uint32_t t = tid - (ND + 192);
+        uint32_t before[2] = {0, 0};       // limbs each buffer holds
+        auto cur = fetch(first);
         for (uint64_t i = first; i < n && ok; i += step, p++) {
+            const auto next = fetch(i + step < n ? i + step : i);
             const uint32_t buf = p % g.NA;
             ok = tc_warp_wait(a_empty + 8 * buf, ((p / g.NA) & 1) ^ 1);
             uint8_t* as = smem + buf * lay.abytes - g.rho0 * 16;
             uint64_t* bs = reinterpret_cast<uint64_t*>(smem + lay.braw + buf * lay.bbytes) + S::PAD;
 #pragma unroll 4
-            for (uint32_t x = t; x < g.L; x += 64) {
-                const uint64_t v = load_a(i, x);
-                bs[x] = load_b(i, x);
+            for (uint32_t x = t; x < cur.L; x += 64) {
+                const uint64_t v = cur.a(x);
+                bs[x] = cur.b(x);
                 const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
                 *reinterpret_cast<uint4*>(as + (x % Q * g.R + x / Q) * 16) =
                     make_uint4(tc_digits(lo, 0x4140), tc_digits(lo, 0x4342), tc_digits(hi, 0x4140), tc_digits(hi, 0x4342));
             }
+            for (uint32_t x = cur.L + t; x < (buf == 0 ? before[0] : before[1]); x += 64) {   // what the last instance had above
+                bs[x] = 0;
+                *reinterpret_cast<uint4*>(as + (x % Q * g.R + x / Q) * 16) = make_uint4(0, 0, 0, 0);
+            }
+            if (buf == 0) before[0] = cur.L;
+            else before[1] = cur.L;
             tc_fence_smem();
             tc_warp_arrive(a_full + 8 * buf);
+            cur = next;
         }
     } else if (warp >= ND / 32) {
         if (warp < ND / 32 + 4) {
@@ -358,13 +368,15 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
             static_assert(NS % 4 == 0, "each stage has one warp");
             const uint32_t t = tid & 31, own = warp - ND / 32, j1 = (t & 7) + 1;
             const uint32_t sel = 0x3210u + 0x1111u * (j1 & 3);
+            auto cur = fetch(first);
             for (uint64_t i = first; i < n && ok; i += step, p++) {
-                const uint32_t buf = p % g.NA;
+                const auto next = fetch(i + step < n ? i + step : i);
+                const uint32_t buf = p % g.NA, D = tc_rows<P>(cur.L), tiles = tc_tiles<P>(cur.out_limbs);
                 ok = tc_warp_wait(a_full + 8 * buf, (p / g.NA) & 1);
                 const uint32_t* bs = reinterpret_cast<const uint32_t*>(smem + lay.braw + buf * lay.bbytes) + 2 * S::PAD + (j1 >> 2);
-                for (uint32_t tau = 0; tau < g.tiles && ok; tau++) {
+                for (uint32_t tau = 0; tau < tiles && ok; tau++) {
                     int klo, khi;
-                    tc_krange(g.D, tau, klo, khi);
+                    tc_krange(D, tau, klo, khi);
                     for (int k0 = klo; k0 <= khi && ok; k0 += S::RB, c++) {
                         if (c % 4 != own) continue;
                         ok = tc_warp_wait(run + 8 * (c % NS), ((c / NS) & 1) ^ 1);
@@ -385,18 +397,21 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
                     }
                 }
                 tc_warp_arrive(a_empty + 8 * buf);     // b's limbs are read
+                cur = next;
             }
         } else {
             // ---- issuing: two warps take the blocks in turn (waiting, the
             // instructions and the commit cost one warp more than the tensor
             // core takes for a block)
             const uint32_t own = warp - (ND / 32 + 4);
+            auto cur = fetch(first);
             for (uint64_t i = first; i < n && ok; i += step, p++) {
-                const uint32_t buf = p % g.NA;
+                const auto next = fetch(i + step < n ? i + step : i);
+                const uint32_t buf = p % g.NA, D = tc_rows<P>(cur.L), tiles = tc_tiles<P>(cur.out_limbs);
                 ok = tc_warp_wait(a_full + 8 * buf, (p / g.NA) & 1);
-                for (uint32_t tau = 0; tau < g.tiles && ok; tau++) {
+                for (uint32_t tau = 0; tau < tiles && ok; tau++) {
                     int klo, khi;
-                    tc_krange(g.D, tau, klo, khi);
+                    tc_krange(D, tau, klo, khi);
                     const uint32_t row0 = (sbase + buf * lay.abytes) / 16 + (uint32_t)((int)(128 * tau) - g.rho0);
                     for (int k0 = klo; k0 <= khi && ok; k0 += S::RB, c++) {
                         if (c % 2 != own) continue;
@@ -416,6 +431,7 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
                 }
                 if (ok && tc_elect()) tc_commit(a_empty + 8 * buf);
                 __syncwarp();
+                cur = next;
             }
             // no matrix instruction is in flight when the tensor memory is freed
             if (tc_elect()) tc_commit(done);
@@ -431,11 +447,14 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
         const uint32_t tbase = tmem + (((warp & 3) * 32) << 16) + (warp >> 2) * CT;
         const uint32_t sg = (tid & 127) * S::H + (S::H - 1 - (warp >> 2));
         // (after a wait ran out: on without waiting, in step for the barriers, storing nothing)
+        auto cur = fetch(first);
         for (uint64_t i = first; i < n; i += step) {
+            const auto next = fetch(i + step < n ? i + step : i);
+            const uint32_t D = tc_rows<P>(cur.L), tiles = tc_tiles<P>(cur.out_limbs);
             if (tid == 0) ovf[0] = 0;
-            for (uint32_t tau = 0; tau < g.tiles; tau++) {
+            for (uint32_t tau = 0; tau < tiles; tau++) {
                 int klo, khi;
-                tc_krange(g.D, tau, klo, khi);
+                tc_krange(D, tau, klo, khi);
                 uint32_t acc[CT], bias = 0;
 #pragma unroll
                 for (int j = 0; j < CT; j++) acc[j] = 0;
@@ -499,10 +518,11 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
                 }
                 asm volatile("bar.sync 1, %0;" ::"r"(ND) : "memory");
                 const uint32_t x0 = tau * 128 * Q;
-                for (uint32_t idx = tid; ok && idx < 128 * Q && x0 + idx < g.out_limbs; idx += ND)
-                    store(i, x0 + idx, rows[idx + idx / QT]);
+                for (uint32_t idx = tid; ok && idx < 128 * Q && x0 + idx < cur.out_limbs; idx += ND)
+                    cur.store(x0 + idx, rows[idx + idx / QT]);
                 asm volatile("bar.sync 1, %0;" ::"r"(ND) : "memory");
             }
+            cur = next;
         }
     }
     if (!ok) atomicAdd(gave_up, 1u);

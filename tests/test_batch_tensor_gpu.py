@@ -79,3 +79,42 @@ def test_division_classes(bigint, copies):
                                       fl.data_ptr(), fl.numel(), None)
     assert st == 0
     _check(words, d, B.to_host(aout, np.uint64), fl.cpu().numpy())
+
+
+@pytest.mark.parametrize("n", [40, 600])
+def test_multiply_classes(bigint, n):
+    """Full and truncated products on both sides of each tensor-core class,
+    largest and smallest in one launch, so that a buffer holds a smaller operand
+    after a larger one."""
+    import torch
+
+    B = bigint
+    rng = random.Random(n)
+    edges = [150, 159, 160, 161, 207, 208, 256, 257, 300, 512, 513, 700, 1024, 1025, 2048]
+    descs, nin, nout = [], 0, 0
+    for k in range(n):
+        full = k % 3 != 2
+        w = 32 if k % 4 == 3 else 64
+        m = edges[k % len(edges)] if k < 2 * len(edges) else rng.randint(140, 700)
+        e = 64 // w
+        mm = m * e - (w == 32 and k % 8 == 3)
+        rl = (2 if full else 1) * m
+        descs.append((B.OP_MULFULL if full else B.OP_MUL, mm, mm, w, nin * e, (nin + m) * e, nout * e, 0, 0))
+        nin += 2 * m
+        nout += rl
+    d = np.array(descs, dtype=B.DESC_DTYPE)
+    words = np.random.default_rng(n).integers(0, 1 << 64, nin, dtype=np.uint64)
+    words[: nin // 8] = np.uint64(0xFFFFFFFFFFFFFFFF)
+    ain = B.to_device(words)
+    aout = torch.zeros(nout, dtype=torch.int64, device="cuda")
+    plan = B.Plan(d, nin, nout)
+    for _ in range(2):
+        plan.execute(ain, aout)
+    torch.cuda.synchronize()
+    out = B.to_host(aout, np.uint64)
+    for x in d:
+        w, m, full = int(x["width"]), int(x["m"]), int(x["op"]) == B.OP_MULFULL
+        u, v = _val(words, int(x["a"]), m, w), _val(words, int(x["b"]), m, w)
+        k = 2 * m if full else m
+        assert _val(out, int(x["r"]), k, w) == u * v % (1 << (w * k)), tuple(x)
+    plan.close()
