@@ -124,6 +124,8 @@ bi_status check_launch(const char* what);
 int num_sms();
 cudaError_t smem_opt_in(const void* func, size_t smem);
 int tc_ctas_per_sm(const void* kern, uint32_t threads, size_t smem, uint32_t cols);
+// products of at most 160 (full) or 256 (truncated) limbs, one warp each (mulmma.cu)
+bi_status mul_mma(const void* a, const void* b, void* r, uint32_t m, uint64_t n, bool w32, bool full, cudaStream_t st);
 // add/sub on pinned host buffers read over the CPU-GPU link (addsub.cu)
 bi_status add_link_u64(const uint64_t* a, const uint64_t* b, uint64_t* r, uint32_t m, uint64_t n, bi_stream s);
 bi_status add_link_u32(const uint32_t* a, const uint32_t* b, uint32_t* r, uint32_t m, uint64_t n, bi_stream s);

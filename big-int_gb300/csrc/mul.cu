@@ -443,21 +443,34 @@ static bi_status mul_tc(const T* a, const T* b, T* r, uint32_t m, uint64_t n, cu
 
 constexpr uint32_t MUL_MAX_L = 4096;   // u64-view limbs per operand
 
-// Products on the tensor cores: the largest sizes always; down to 33 limbs
-// while a batch is a few CTAs an SM.  Measured against the CTA kernel's best
-// tiling (u64): full products of 192 / 256 / 512 / 1024 / 2048 / 4096 limbs
-// 1.43 / 1.84 / 2.82 / 4.18 / 4.13 / 6.0 times its rate at 2^22 limbs an
-// operand, of 128 limbs 0.95; truncated ones of 250 / 512 / 1024 / 2048 limbs
-// 1.22 / 2.05 / 3.03 / 4.59, of 192 limbs 0.92.  With 8 instances an SM or
-// fewer one instance's serial rows bound the CTA kernel: 64 limbs 4.5 us
-// against 12.7 with one instance, 11.5 against 13.9 with 1216; 1024 limbs
-// 26.9 against 146.
-constexpr uint32_t MUL_TC_MIN_L = 33, MUL_TC_FULL_L = 160, MUL_TC_TRUNC_L = 208, MUL_TC_SM_INSTANCES = 8;
+// Which products the tensor cores take (u64, us, before / there; the thread,
+// warp and CTA kernels' best tiling before).
+//   multc.cuh: above 160 limbs (full) or 256 (truncated).  Full products of 192
+//   limbs 581 / 406 (21845 of them), 256 722 / 391, 512 1369 / 485, 1024 2655 /
+//   628, 4096 10650 / 1776; truncated ones of 320 483 / 382, 1024 1394 / 460.
+//   mulmma.cuh, one warp an instance: below.  Full products of 33 limbs 157 / 100
+//   (65536), 64 237 / 118, 96 340 / 172 (43690), 128 395 / 180 (32768), 160 513 /
+//   260 (26214); truncated ones of 64 133 / 81, 128 215 / 105, 256 383 / 214.
+//   One instance an SM or fewer: the wider multc.cuh is a little faster from
+//   about 100 limbs (192 truncated) on: 160 limbs 8.4 / 6.3.
+//   Up to 32 limbs the thread kernel wins as soon as the batch is large enough
+//   for one thread an instance; until then a thread's serial product is what
+//   takes the time: 24 limbs 12.2 / 2.6 us (one), 13.7 / 10.0 (9728), 13.9 / 17.9
+//   (19456); 16 limbs 6.9 / 4.5 (4864); 8 limbs 3.5 / 3.4 (2432).  From 25 to 32
+//   limbs (full) the warp kernel is as fast up to 8 an SM, 67 / 59 at 65536.
+enum { MUL_OTHER = 0, MUL_TC = 1, MUL_MMA = 2 };
 
-static bool mul_use_tc(uint32_t L, bool full, uint64_t n) {
-    if (L >= (full ? MUL_TC_FULL_L : MUL_TC_TRUNC_L)) return true;
-    return L >= MUL_TC_MIN_L && n <= (uint64_t)MUL_TC_SM_INSTANCES * num_sms();
+static int mul_matrix_kernel(uint32_t L, bool full, uint64_t n) {
+    const uint64_t sms = (uint64_t)num_sms();
+    if (L > (full ? 160u : 256u)) return MUL_TC;
+    if (n <= sms && L > (full ? 96u : 192u)) return MUL_TC;
+    if (L > 32) return MUL_MMA;
+    if (L < 8) return MUL_OTHER;
+    if (full && L > MUL_THREAD_MAX_L) return n > 8 * sms ? MUL_MMA : MUL_OTHER;
+    const uint64_t per_sm = full ? (L < 12 ? 16 : L < 16 ? 32 : 64) : (L < 12 ? 8 : L < 16 ? 16 : L < 24 ? 32 : 64);
+    return n <= per_sm * sms ? MUL_MMA : MUL_OTHER;
 }
+
 constexpr uint32_t MUL_WARP_MAX_L = 32;    // full products above MUL_THREAD_MAX_L up to here: the warp kernel
 
 // ---------------------------------------------------------------------------
@@ -535,26 +548,38 @@ static bi_status mul_launch_geom(const T* a, const T* b, T* r, uint32_t m, uint6
     return check_launch(FULL ? "mulfull kernel" : "mul kernel");
 }
 
+// mul_matrix_kernel's kernel `kind`
+template <typename T, bool FULL>
+static bi_status mul_matrix(int kind, const T* a, const T* b, T* r, uint32_t m, uint64_t n, cudaStream_t st) {
+    if constexpr (sizeof(T) == 4) {
+        // an even word count on 8-byte-aligned buffers: the same bytes as m/2 64-bit limbs
+        if (m % 2 == 0 && ((uintptr_t)a | (uintptr_t)b | (uintptr_t)r) % 8 == 0)
+            return mul_matrix<uint64_t, FULL>(kind, reinterpret_cast<const uint64_t*>(a), reinterpret_cast<const uint64_t*>(b),
+                                              reinterpret_cast<uint64_t*>(r), m / 2, n, st);
+    }
+    if (kind == MUL_MMA) return mul_mma(a, b, r, m, n, sizeof(T) == 4, FULL, st);
+    return mul_tc<T, FULL>(a, b, r, m, n, st);
+}
+
 template <typename T, bool FULL>
 static bi_status mul_launch(const T* a, const T* b, T* r, uint32_t m, uint64_t n, cudaStream_t st) {
     const uint32_t L = sizeof(T) == 8 ? m : (m + 1) / 2;
     if (L > MUL_MAX_L) return set_error(BI_EUNSUPPORTED, "mul: m=%u above the supported size", m);
     constexpr uint32_t THREAD_MAX = FULL ? MUL_THREAD_MAX_L : MUL_THREAD_TRUNC_MAX_L;
+    MulTune t;
+    const bool tuned = mul_tuning_lookup((int)sizeof(T), FULL, L, &t);
+    const int kind = mul_matrix_kernel(L, FULL, n);
+    if (!tuned && kind != MUL_OTHER) return mul_matrix<T, FULL>(kind, a, b, r, m, n, st);
     if (L <= THREAD_MAX || (FULL && L <= MUL_WARP_MAX_L)) {
         // the thread kernel (L <= MUL_THREAD_MAX_L) or, for full products, the
         // warp kernel, unless a tuning picked one of them ({0, 1}, {0, 0}) or
         // a CTA tiling
-        MulTune t;
-        const bool tuned = mul_tuning_lookup((int)sizeof(T), FULL, L, &t);
         if (!tuned || t.ipc == 0) {
             const bool thread = tuned ? t.S == 1 : L <= THREAD_MAX;
             if (thread) return mul_thread<T, FULL>(a, b, r, m, n, st);
             if constexpr (FULL) return mul_warp<T>(a, b, r, m, n, st);
         }
     }
-    MulTune t;
-    if (mul_use_tc(L, FULL, n) && !mul_tuning_lookup((int)sizeof(T), FULL, L, &t))
-        return mul_tc<T, FULL>(a, b, r, m, n, st);
     return mul_launch_geom<T, FULL>(a, b, r, m, n, mul_geom_for<T, FULL>(L, n), st);
 }
 
@@ -604,8 +629,8 @@ static bi_status mul_chain(const T* a, const T* b, T* r, uint32_t m, uint64_t n,
 // as {0, 1}, beside the CTA
 // kernel's tilings (64-bit limbs: row_mac8) -- the arithmetic's word width
 // and the threads an instance are part of what is tuned.  Where the call
-// would go to the tensor cores they are a candidate too: one instance a CTA,
-// {1, 1}, and nothing is recorded when they are the fastest.
+// would go to the tensor cores they are a candidate too, reported as {1, 1}, and
+// nothing is recorded when they are the fastest.
 template <typename T, bool FULL>
 static bi_status mul_autotune(const T* a, const T* b, T* r, uint32_t m, uint64_t n, int reps, int* chosen,
                               cudaStream_t st) {
@@ -638,17 +663,17 @@ static bi_status mul_autotune(const T* a, const T* b, T* r, uint32_t m, uint64_t
     float best = 1e30f;
     MulTune pick = {cands[0].first, cands[0].second};
     bi_status st_out = BI_OK;
-    const bool tc = mul_use_tc(L, FULL, n);
+    const int kind = mul_matrix_kernel(L, FULL, n);
     const size_t ntiled = cands.size();
-    if (tc) cands.push_back({1, 1});
-    bool pick_tc = false;
+    if (kind != MUL_OTHER) cands.push_back({1, 1});
+    bool pick_matrix = false;
     for (size_t ci = 0; ci < cands.size(); ci++) {
         const auto& c = cands[ci];
-        const bool on_tc = ci >= ntiled;
+        const bool on_matrix = ci >= ntiled;
         std::vector<float> ts;
         for (int k = 0; k <= reps && st_out == BI_OK; k++) {   // the first run warms up
             cudaEventRecord(e0, st);
-            st_out = on_tc ? mul_tc<T, FULL>(a, b, r, m, n, st) : run(c.first, c.second);
+            st_out = on_matrix ? mul_matrix<T, FULL>(kind, a, b, r, m, n, st) : run(c.first, c.second);
             cudaEventRecord(e1, st);
             if (cudaEventSynchronize(e1) != cudaSuccess) st_out = set_error(BI_ECUDA, "mul autotune: %s",
                                                                             cudaGetErrorString(cudaGetLastError()));
@@ -662,7 +687,7 @@ static bi_status mul_autotune(const T* a, const T* b, T* r, uint32_t m, uint64_t
         if (med < best) {
             best = med;
             pick = {c.first, c.second};
-            pick_tc = on_tc;
+            pick_matrix = on_matrix;
         }
     }
     cudaEventDestroy(e0);
@@ -673,11 +698,11 @@ static bi_status mul_autotune(const T* a, const T* b, T* r, uint32_t m, uint64_t
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         const auto key = std::make_tuple(dev, (int)sizeof(T), FULL ? 1 : 0, L);
-        if (pick_tc) g_tune.erase(key);    // the library's own choice
+        if (pick_matrix) g_tune.erase(key);    // the library's own choice
         else g_tune[key] = pick;
     }
     // leave r as one plain call with the chosen tiling writes it
-    BI_RETURN_IF((pick_tc ? mul_tc<T, FULL>(a, b, r, m, n, st) : run(pick.ipc, pick.S)));
+    BI_RETURN_IF((pick_matrix ? mul_matrix<T, FULL>(kind, a, b, r, m, n, st) : run(pick.ipc, pick.S)));
     if (chosen) {
         chosen[0] = (int)pick.ipc;
         chosen[1] = (int)pick.S;

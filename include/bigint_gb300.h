@@ -106,12 +106,13 @@ bi_status bi_mulfull_u32(const uint32_t* a, const uint32_t* b, uint32_t* r,
                          uint32_t m, uint64_t n, bi_stream stream);
 
 /* Tiling of the CTA multiply (64-bit limb arithmetic): instances per CTA */
-/* and row slices per window pair. Full products of at most 24 64-bit     */
-/* limbs and truncated ones of at most 32 run by default on the thread    */
-/* kernel (one thread an instance, 64-bit limbs), full products of 25 to  */
-/* 32 limbs on the warp kernel (32-bit words); full products of at least  */
-/* 160 limbs, truncated ones of at least 208 and, in small batches, those */
-/* of 33 limbs on run on the tensor cores.  bi_mul_autotune_* times       */
+/* and row slices per window pair. Products above 32 64-bit limbs run by  */
+/* default on the tensor cores (one warp an instance up to 160 limbs full, */
+/* 256 truncated, CTAs above).  Up to there full products of at most 24    */
+/* limbs and truncated ones run on the thread kernel (one thread an        */
+/* instance, 64-bit limbs) and full products of 25 to 32 limbs on the warp */
+/* kernel (32-bit words), or on the tensor cores where n is too small for  */
+/* the first or large for the second.  bi_mul_autotune_* times             */
 /* every tiling that fits on the caller's a, b -- and the warp kernel for */
 /* full products of at most 32 64-bit limbs, the thread kernel where it   */
 /* takes the size -- (median of `reps` runs each), records the fastest    */
