@@ -224,6 +224,7 @@ constexpr int DIV_BLK2_CLASS = DIV_CTA_CLASS + 1, DIV_BLK4_CLASS = DIV_CTA_CLASS
 // width, for the divisions of batch_div_on_tc
 constexpr int DIV_TC_CLASSES = 5, DIV_TC0 = DIV_CTA_CLASS + 3;
 constexpr int DIV_TC_P[DIV_TC_CLASSES] = {16, 32, 64, 80, 128};
+constexpr int DIV_TC_G[DIV_TC_CLASSES] = {1, 1, 1, 2, 1};   // as the uniform entry's for full batches
 constexpr int DIV_CLASSES = DIV_TC0 + DIV_TC_CLASSES;
 constexpr int DIV_CTA_THREADS = 512;
 // add/sub, multiply, one per division class, one per warp-multiply class
@@ -236,13 +237,13 @@ constexpr int PLAN_MULTC0 = PLAN_MULW0 + MULW_CLASSES;   // and of the first ten
 // setup (div.cu's rule for a batch that fills the GPU; up to 128 limbs the
 // lane groups pack better beside the batch's other kernels).
 static inline bool batch_div_on_tc(uint32_t m, uint32_t mv) {
-    return mv > 128 && mv <= (uint32_t)DtShape<128>::MAX_K && (uint64_t)mv * (m - mv + 1) >= 9400;
+    return mv > 128 && mv <= (uint32_t)DtShape<128, 1>::MAX_K && (uint64_t)mv * (m - mv + 1) >= 9400;
 }
 
 static inline int div_class(uint32_t m, uint32_t mv) {
     if (batch_div_on_tc(m, mv)) {
         int c = 0;
-        while (mv > 16u * DIV_TC_P[c] - DT_KB - 2) c++;
+        while (mv > 16u * DIV_TC_P[c] - (32u * DIV_TC_G[c] - 1) - 2) c++;
         return DIV_TC0 + c;
     }
     if (mv <= 4) return 0;
@@ -456,15 +457,15 @@ batch_divblk_kernel(const bi_desc* __restrict__ descs, const uint32_t* __restric
 
 // Divisions in blocks on the tensor cores (divtc.cuh), one at a time a CTA;
 // `mu` sizes the window for the class's largest dividend.
-template <int P>
-__global__ void __launch_bounds__(DtShape<P>::NT)
+template <int P, int G>
+__global__ void __launch_bounds__(DtShape<P, G>::NT)
 batch_divtc_kernel(const bi_desc* __restrict__ descs, const uint32_t* __restrict__ list, uint32_t count,
                    uint32_t* counter, const uint64_t* in, uint64_t* out, uint8_t* flags, uint32_t mu) {
     extern __shared__ __align__(128) uint8_t smem_dt[];
     __shared__ uint32_t s_idx;
-    const DtSmem<P> lay(dt_geom(mu, 1, 8));
+    const DtSmem<P, G> lay(dt_geom(mu, 1, 8));
     const uint32_t bar = tc_smem_addr(smem_dt) + lay.bar;
-    const uint32_t tmem = tc_alloc<DtShape<P>::TMEM_COLS>(bar + 8, [&] { tc_bar_init(bar, 1); });
+    const uint32_t tmem = tc_alloc<DtShape<P, G>::TMEM_COLS>(bar + 8, [&] { tc_bar_init(bar, 1); });
     uint32_t phase = 0;
     for (;;) {
         if (threadIdx.x == 0) s_idx = atomicAdd(counter, 1u);
@@ -478,10 +479,10 @@ batch_divtc_kernel(const bi_desc* __restrict__ descs, const uint32_t* __restrict
         auto lv = [&](uint32_t i) { return ld64(in, d.b, d.mb, w32, i); };
         auto sq = [&](uint32_t i, uint64_t x) { st64(out, d.r, d.m, w32, i, x); };
         auto sr = [&](uint32_t i, uint64_t x) { st64(out, d.r2, d.mb, w32, i, x); };
-        const uint8_t st = dt_divide<P>(dt_geom(m64(d), mb64(d), 8), lay, smem_dt, tmem, phase, lu, lv, sq, sr);
+        const uint8_t st = dt_divide<P, G>(dt_geom(m64(d), mb64(d), 8), lay, smem_dt, tmem, phase, lu, lv, sq, sr);
         if (flags && threadIdx.x == 0) flags[d.flag] = st;
     }
-    tc_free<DtShape<P>::TMEM_COLS>(tmem);
+    tc_free<DtShape<P, G>::TMEM_COLS>(tmem);
 }
 
 struct bi_plan {
@@ -585,11 +586,11 @@ static bool div_before(const bi_desc& x, const bi_desc& y, const int* map) {
 static size_t div_tc_smem(int k, uint32_t mu) {
     const DtGeom g = dt_geom(mu, 1, 8);
     switch (k) {
-    case 0: return DtSmem<16>(g).total;
-    case 1: return DtSmem<32>(g).total;
-    case 2: return DtSmem<64>(g).total;
-    case 3: return DtSmem<80>(g).total;
-    default: return DtSmem<128>(g).total;
+    case 0: return DtSmem<16, 1>(g).total;
+    case 1: return DtSmem<32, 1>(g).total;
+    case 2: return DtSmem<64, 1>(g).total;
+    case 3: return DtSmem<80, 2>(g).total;
+    default: return DtSmem<128, 1>(g).total;
     }
 }
 
@@ -636,11 +637,11 @@ static const void* div_class_kernel(int c, int* threads) {
                : c == DIV_BLK2_CLASS ? 64 : c == DIV_BLK4_CLASS ? 128
                : c < DIV_TC0 ? DIV_CTA_THREADS : DIV_TC_P[c - DIV_TC0] >= 80 ? 256 : 128;
     switch (c) {
-    case DIV_TC0: return (const void*)batch_divtc_kernel<16>;
-    case DIV_TC0 + 1: return (const void*)batch_divtc_kernel<32>;
-    case DIV_TC0 + 2: return (const void*)batch_divtc_kernel<64>;
-    case DIV_TC0 + 3: return (const void*)batch_divtc_kernel<80>;
-    case DIV_TC0 + 4: return (const void*)batch_divtc_kernel<128>;
+    case DIV_TC0: return (const void*)batch_divtc_kernel<16, 1>;
+    case DIV_TC0 + 1: return (const void*)batch_divtc_kernel<32, 1>;
+    case DIV_TC0 + 2: return (const void*)batch_divtc_kernel<64, 1>;
+    case DIV_TC0 + 3: return (const void*)batch_divtc_kernel<80, 2>;
+    case DIV_TC0 + 4: return (const void*)batch_divtc_kernel<128, 1>;
     case DIV_BLK2_CLASS: return (const void*)batch_divblk_kernel<2>;
     case DIV_BLK4_CLASS: return (const void*)batch_divblk_kernel<4>;
     case 0: return (const void*)batch_divthread_kernel<4>;
@@ -832,11 +833,11 @@ static bi_status launch_plan_kernels(bi_plan* p, const uint64_t* in, uint64_t* o
             case 8: batch_divwarp_kernel<16><<<grid, DIV_WARP_CTA, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             case 9: batch_divwarp3_kernel<24><<<grid, DIV_WARP_CTA, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             case 10: batch_divwarp_kernel<32><<<grid, DIV_WARP_CTA, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
-            case DIV_TC0: batch_divtc_kernel<16><<<grid, DtShape<16>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[0]); break;
-            case DIV_TC0 + 1: batch_divtc_kernel<32><<<grid, DtShape<32>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[1]); break;
-            case DIV_TC0 + 2: batch_divtc_kernel<64><<<grid, DtShape<64>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[2]); break;
-            case DIV_TC0 + 3: batch_divtc_kernel<80><<<grid, DtShape<80>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[3]); break;
-            case DIV_TC0 + 4: batch_divtc_kernel<128><<<grid, DtShape<128>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[4]); break;
+            case DIV_TC0: batch_divtc_kernel<16, 1><<<grid, DtShape<16, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[0]); break;
+            case DIV_TC0 + 1: batch_divtc_kernel<32, 1><<<grid, DtShape<32, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[1]); break;
+            case DIV_TC0 + 2: batch_divtc_kernel<64, 1><<<grid, DtShape<64, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[2]); break;
+            case DIV_TC0 + 3: batch_divtc_kernel<80, 2><<<grid, DtShape<80, 2>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[3]); break;
+            case DIV_TC0 + 4: batch_divtc_kernel<128, 1><<<grid, DtShape<128, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[4]); break;
             case DIV_BLK2_CLASS: batch_divblk_kernel<2><<<grid, 64, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             case DIV_BLK4_CLASS: batch_divblk_kernel<4><<<grid, 128, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             default:

@@ -283,45 +283,45 @@ static void launch_div_blk(const T* u, const T* v, T* q, T* r, uint8_t* status, 
 }
 
 // ---------------------------------------------------------------------------
-// Long division 31 quotient limbs at a time on the tensor cores (divtc.cuh),
-// one instance a CTA at a time, the CTAs persistent.  2048 divisions of 2048
-// by 1024 limbs 3400 -> 626 us, 8192 of 512 by 256 1013 -> 409: a quotient
-// block's chain -- estimate, product, fold, carries -- is about 6K cycles of
-// latency with four CTAs an SM (issue slots 45 % busy), of which the matrix
-// instructions are 1.1K at 1024 limbs.
+// Long division 31 or 63 quotient limbs at a time on the tensor cores
+// (divtc.cuh), one instance a CTA at a time, the CTAs persistent.  2048
+// divisions of 2048 by 1024 limbs 3400 -> 565 us, 8192 of 512 by 256 1013 ->
+// 409.  Bound by the latency of a block's chain -- estimate, product, fold,
+// carries, each behind a barrier: issue slots 45 % busy at four CTAs an SM (what
+// tensor memory holds at 1024 limbs), the tensor core about 40 %.
 // ---------------------------------------------------------------------------
-template <typename T, int P>
-__global__ void __launch_bounds__(DtShape<P>::NT)
+template <typename T, int P, int G>
+__global__ void __launch_bounds__(DtShape<P, G>::NT)
 div_tc_kernel(const T* __restrict__ u, const T* __restrict__ v, T* __restrict__ q, T* __restrict__ r,
               uint8_t* __restrict__ status, uint64_t n, DtGeom g) {
     extern __shared__ __align__(128) uint8_t smem_dt[];
-    const DtSmem<P> lay(g);
+    const DtSmem<P, G> lay(g);
     const uint32_t bar = tc_smem_addr(smem_dt) + lay.bar;
-    const uint32_t tmem = tc_alloc<DtShape<P>::TMEM_COLS>(bar + 8, [&] { tc_bar_init(bar, 1); });
+    const uint32_t tmem = tc_alloc<DtShape<P, G>::TMEM_COLS>(bar + 8, [&] { tc_bar_init(bar, 1); });
     uint32_t phase = 0;
     for (uint64_t inst = blockIdx.x; inst < n; inst += gridDim.x) {
         const T* ui = u + inst * g.mu;
         const T* vi = v + inst * g.mv;
         T* qi = q + inst * g.mu;
         T* ri = r + inst * g.mv;
-        const uint8_t st = dt_divide<P>(
+        const uint8_t st = dt_divide<P, G>(
             g, lay, smem_dt, tmem, phase, [&](uint32_t i) { return limb64(ui, g.mu, i); },
             [&](uint32_t i) { return limb64(vi, g.mv, i); }, [&](uint32_t i, uint64_t x) { put_limb64(qi, g.mu, i, x); },
             [&](uint32_t i, uint64_t x) { put_limb64(ri, g.mv, i, x); });
         if (status && threadIdx.x == 0) status[inst] = st;
     }
-    tc_free<DtShape<P>::TMEM_COLS>(tmem);
+    tc_free<DtShape<P, G>::TMEM_COLS>(tmem);
 }
 
-template <typename T, int P>
+template <typename T, int P, int G>
 static bi_status launch_div_tc(const T* u, const T* v, T* q, T* r, uint8_t* status, uint64_t n, const DtGeom& g,
                                cudaStream_t s) {
-    const size_t smem = DtSmem<P>(g).total;
-    auto kern = div_tc_kernel<T, P>;
+    const size_t smem = DtSmem<P, G>(g).total;
+    auto kern = div_tc_kernel<T, P, G>;
     cudaError_t e = smem_opt_in((const void*)kern, smem);
     if (e != cudaSuccess) return set_error(BI_ECUDA, "div: %s", cudaGetErrorString(e));
-    const uint64_t cap = (uint64_t)num_sms() * tc_ctas_per_sm((const void*)kern, DtShape<P>::NT, smem, DtShape<P>::TMEM_COLS);
-    kern<<<(unsigned)(n < cap ? n : cap), DtShape<P>::NT, smem, s>>>(u, v, q, r, status, n, g);
+    const uint64_t cap = (uint64_t)num_sms() * tc_ctas_per_sm((const void*)kern, DtShape<P, G>::NT, smem, DtShape<P, G>::TMEM_COLS);
+    kern<<<(unsigned)(n < cap ? n : cap), DtShape<P, G>::NT, smem, s>>>(u, v, q, r, status, n, g);
     return check_launch("div tensor kernel");
 }
 
@@ -330,12 +330,17 @@ template <typename T>
 static bi_status div_tc(const T* u, const T* v, T* q, T* r, uint8_t* status, uint32_t mu, uint32_t mv, uint64_t n,
                         cudaStream_t s) {
     const DtGeom g = dt_geom(mu, mv, (int)sizeof(T));
-    if (g.MV <= (uint32_t)DtShape<16>::MAX_K) return launch_div_tc<T, 16>(u, v, q, r, status, n, g, s);
-    if (g.MV <= (uint32_t)DtShape<32>::MAX_K) return launch_div_tc<T, 32>(u, v, q, r, status, n, g, s);
-    if (g.MV <= (uint32_t)DtShape<48>::MAX_K) return launch_div_tc<T, 48>(u, v, q, r, status, n, g, s);
-    if (g.MV <= (uint32_t)DtShape<64>::MAX_K) return launch_div_tc<T, 64>(u, v, q, r, status, n, g, s);
-    if (g.MV <= (uint32_t)DtShape<80>::MAX_K) return launch_div_tc<T, 80>(u, v, q, r, status, n, g, s);
-    return launch_div_tc<T, 128>(u, v, q, r, status, n, g, s);
+    if (g.MV <= (uint32_t)DtShape<16, 1>::MAX_K) return launch_div_tc<T, 16, 1>(u, v, q, r, status, n, g, s);
+    if (g.MV <= (uint32_t)DtShape<32, 1>::MAX_K) return launch_div_tc<T, 32, 1>(u, v, q, r, status, n, g, s);
+    if (g.MV <= (uint32_t)DtShape<48, 1>::MAX_K) return launch_div_tc<T, 48, 1>(u, v, q, r, status, n, g, s);
+    if (g.MV <= (uint32_t)DtShape<64, 1>::MAX_K) return launch_div_tc<T, 64, 1>(u, v, q, r, status, n, g, s);
+    // blocks of 63 limbs: 2048 divisions of 2048 by 1024 limbs 627 -> 565 us, one
+    // 87 -> 72; of 3072 by 1536 one 159 -> 119 us, 1365 of them 1013 -> 1052;
+    // below 992 limbs slower (512: 435 -> 477 at 4096 of them)
+    if (g.MV <= (uint32_t)DtShape<80, 2>::MAX_K) return launch_div_tc<T, 80, 2>(u, v, q, r, status, n, g, s);
+    if (n <= (uint64_t)num_sms() && g.MV <= (uint32_t)DtShape<128, 2>::MAX_K)
+        return launch_div_tc<T, 128, 2>(u, v, q, r, status, n, g, s);
+    return launch_div_tc<T, 128, 1>(u, v, q, r, status, n, g, s);
 }
 
 // Measured against the lane groups, the warps and the shifted inverse (us, u64,
@@ -351,7 +356,7 @@ static bi_status div_tc(const T* u, const T* v, T* q, T* r, uint8_t* status, uin
 // 18; 2432 with m = 72 61 / 54, with m = 64 50 / 54.
 static bool div_use_tc(uint32_t MU, uint32_t MV, uint64_t n) {
     const uint64_t ql = MU - MV + 1, sms = (uint64_t)num_sms();
-    if (MV < 40 || MV > (uint32_t)DtShape<128>::MAX_K) return false;
+    if (MV < 40 || MV > (uint32_t)DtShape<128, 1>::MAX_K) return false;
     if (MV >= 65 && MV * ql >= 9400) return true;
     return (ql >= 20 && n <= 4 * sms) || (MV >= 65 && ql >= 48 && n <= 16 * sms);
 }

@@ -1,12 +1,12 @@
-// divtc.cuh -- long division by medium and large divisors, DT_KB quotient
+// divtc.cuh -- long division by medium and large divisors, 31 or 63 quotient
 // limbs at a time, the quotient block times the divisor on the tensor cores.
 //
 // One CTA divides one instance; the running remainder ("window")
 // lies in shared memory, the divisor as f16 digits in the Toeplitz layout of
 // multc.cuh, written once per instance.  Per block of quotient limbs:
-//   estimate  q^ = the top 32 window limbs times the 32-limb reciprocal of the
-//             divisor's top 32 limbs (Barrett), the upper half of a 32-by-32
-//             limb product over the CTA's threads;
+//   estimate  q^ = the top LW = 32 or 64 window limbs times the LW-limb
+//             reciprocal of the divisor's top LW limbs (Barrett), the upper
+//             half of an LW-by-LW limb product over the CTA's threads;
 //   product   q^ V as a digit convolution: q^'s core matrices in shared
 //             memory, then one chain of matrix instructions;
 //   subtract  each thread folds its accumulator row with its window limbs, one
@@ -15,15 +15,17 @@
 //             one too large, two too small; both take chance 2^-58 or so on
 //             random operands) is corrected with the whole CTA.
 // Digits are balanced, in [-128, 127]: byte k of x + 0x8080..80 less 128.  A
-// column then sums at most 249 products (q^ has 31 limbs and a carry digit) of
-// magnitude 2^14 at most, below 2^22, so that one accumulator holds a whole
-// block exactly and 1.5 2^23 + v has v in its low bits.
+// column then sums at most 249 or 505 products (q^ has LW - 1 limbs and a carry
+// digit) of magnitude 2^14 at most, below 2^22 or 2^23: one accumulator holds a
+// whole block exactly.  Blocks of 63 limbs halve what a block costs whatever its
+// size -- the fold and the carries over the whole window, the barriers -- and
+// pay for it with a longer reciprocal and four times the estimate's products.
 //
-// With W < V B^31, V's top bit set and K >= 32 limbs, Wt and Vh the top 32
-// limbs of W (K + 31 limbs) and V and I = floor((B^64 - 1) / Vh): q^ =
-// floor((floor(Wt (I - B^32) / B^32) + Wt) / B) differs from floor(W / V) by at
+// With W < V B^(LW-1), V's top bit set and K >= LW limbs, Wt and Vh the top LW
+// limbs of W (K + LW - 1 limbs) and V and I = floor((B^2LW - 1) / Vh): q^ =
+// floor((floor(Wt (I - B^LW) / B^LW) + Wt) / B) differs from floor(W / V) by at
 // most one either way, and by one more below for the columns of the product
-// that are left out.  A divisor of fewer than 32 limbs is scaled by B^(32-K),
+// that are left out.  A divisor of fewer than LW limbs is scaled by B^(LW-K),
 // which scales the remainder.
 #pragma once
 
@@ -33,29 +35,30 @@
 
 namespace bi {
 
-constexpr int DT_KB = 31;            // quotient limbs a block
 constexpr uint64_t DT_HALF = 0x8080808080808080ull;
 constexpr int DT_MAX_CORRECTIONS = 4;
 
-template <int P>
+// G: limbs a lane of LW = 32 G
+template <int P, int G>
 struct DtShape {
+    static constexpr int LW = 32 * G, KB = LW - 1;               // reciprocal limbs, quotient limbs a block
     static constexpr int Q = P / 8;                              // limbs a row
     static constexpr int H = P >= 80 ? 2 : 1;                    // threads a row of the accumulator
     static constexpr int NT = 128 * H;                           // threads
     static constexpr int QT = Q / H;                             // limbs a thread
-    static constexpr int T0 = -256;                              // first term: q^'s 249 digits, down to a multiple of 16
+    static constexpr int T0 = -8 * LW;                           // first term: q^'s 8 KB + 1 digits, down to a multiple of 16
     static constexpr int STEPS = (P - T0) / 16;                  // matrix instructions a block
     static constexpr int CM = Q + 2 * STEPS - 1;                 // core matrices of q^
     static constexpr int KMIN = -((-T0 + P - 1) / P);            // row offset of the first term
     static constexpr int R = ((128 - KMIN) + 6) / 8 * 8 + 1;     // rows of the divisor's image, % 8 == 1
-    static constexpr int MAX_K = 128 * Q - DT_KB - 2;            // divisor limbs: the rows hold K + 33
+    static constexpr int MAX_K = 128 * Q - KB - 2;               // divisor limbs: the rows hold K + KB + 2
     static constexpr uint32_t TMEM_COLS = tc_pow2(P);
     // Place of window limb x: threads 8 limbs apart would all meet in the same
     // banks, so that the eight-limb shapes pad one limb after every eight
     // (1671 -> 988 us for 1048 divisions of 4000 by 2000 limbs; the others ran
     // 3-5 % slower with it)
     __host__ __device__ static constexpr int at(int x) { return QT % 8 == 0 ? x + (x >> 3) : x; }
-    static constexpr int QLO = 2 * STEPS - 32, QHI = Q + 1;      // zero limbs below and above q^ that its blocks read
+    static constexpr int QLO = 2 * STEPS - LW, QHI = Q + 1;      // zero limbs below and above q^ that its blocks read
 };
 
 struct DtGeom {
@@ -64,18 +67,18 @@ struct DtGeom {
     uint32_t UL;           // window limbs (places)
 };
 
-template <int P>
+template <int P, int G>
 struct DtSmem {
     uint32_t stage, win, inv, part, qraw, qh, cs, scratch, bar, total;
     __host__ __device__ explicit DtSmem(const DtGeom& g) {
-        using S = DtShape<P>;
+        using S = DtShape<P, G>;
         stage = S::R * S::Q * 16;
         win = stage + S::CM * 128;
         inv = win + g.UL * 8;
-        part = inv + 64 * 8;
-        qraw = part + 3 * S::NT * 8;
-        qh = qraw + (S::QLO + 32 + S::QHI + 1) / 2 * 16;
-        cs = qh + 34 * 8;
+        part = inv + 2 * S::LW * 8;
+        qraw = part + 3 * S::NT * G * 8;
+        qh = qraw + (S::QLO + S::LW + S::QHI + 1) / 2 * 16;
+        cs = qh + (S::LW + 2) * 8;
         scratch = cs + (S::NT + 1) * 8;
         bar = scratch + 3 * 32 * 4;
         total = bar + 16;
@@ -88,7 +91,7 @@ __host__ __device__ inline DtGeom dt_geom(uint32_t mu, uint32_t mv, int wbytes) 
     g.mv = mv;
     g.MU = wbytes == 8 ? mu : (mu + 1) / 2;
     g.MV = wbytes == 8 ? mv : (mv + 1) / 2;
-    g.UL = (g.MU + 64) * 9 / 8 + 2;
+    g.UL = (g.MU + 130) * 9 / 8 + 2;
     g.UL = g.UL / 2 * 2;
     return g;
 }
@@ -129,6 +132,15 @@ __device__ uint32_t dt_addsub(uint64_t* win, int x0, Limb limb, int len, bool su
     return __syncthreads_or(threadIdx.x == NT - 1 && (hi > lo ? c : cin));
 }
 
+// The integer v: below 2^22, 1.5 2^23 + v has it in the low bits (two ALU
+// instructions, where the conversion unit takes a quarter of their rate);
+// below 2^23 the conversion.
+template <int G>
+__device__ __forceinline__ int32_t dt_int(float v) {
+    if constexpr (G == 1) return (int32_t)(__float_as_uint(v + 12582912.0f) - 0x4B400000u);
+    else return __float2int_rn(v);
+}
+
 // carry out of each lane's (g, p), carry-in 0: the carry into the lane, and out of lane 31
 __device__ __forceinline__ uint32_t dt_lane_carry(uint32_t g, uint32_t p, uint32_t& cout) {
     const WarpCarry w = warp_carry_resolve(__ballot_sync(0xffffffffu, g | p), __ballot_sync(0xffffffffu, g), 0);
@@ -156,11 +168,11 @@ __device__ __forceinline__ uint64_t dt_fold(uint64_t lo, uint64_t mid, uint64_t 
 }
 
 // One step of dt_recip: P limbs of y to 2 P.
-template <int P>
+template <int P, int LW>
 __device__ __forceinline__ void dt_recip_step(const uint64_t* v, uint64_t* y, uint64_t* t) {
     const int lane = (int)(threadIdx.x & 31);
-    const uint64_t* V = v + 32 - 2 * P;
-    const uint64_t* Y = y + 32 - P;
+    const uint64_t* V = v + LW - 2 * P;
+    const uint64_t* Y = y + LW - P;
     // column P - 1 + lane of X Y, X's limbs above its top zero, lanes 0 .. P + 1
     auto column = [&](const uint64_t* X, uint64_t& c0, uint64_t& c1, uint32_t& c2) {
         c0 = c1 = 0;
@@ -196,27 +208,144 @@ __device__ __forceinline__ void dt_recip_step(const uint64_t* v, uint64_t* y, ui
     if (2 * P < 32) over = __shfl_sync(0xffffffffu, cy, (2 * P) & 31);
     if (over) r = pos ? 0 : ~0ull;
     __syncwarp();
-    if (in) y[32 - 2 * P + lane] = r;
+    if (in) y[LW - 2 * P + lane] = r;
     __syncwarp();
 }
 
-// y[0..32) = about floor((B^64 - 1) / V) - B^32 for V = v[0..32), top bit set,
-// v[32] = 0, by one warp: Newton's iteration from the top limb's reciprocal,
-// y + 1 = x -> x + x (1 - V x), with 1, 2, .. 16 limbs of y giving twice as
-// many.  The top halves of 1 - V x cancel and the lowest columns are left out:
-// within 2^24 units of the last limb in 3000 random and extreme divisors,
-// which moves a quotient block by one with a chance of 2^-40.  `t`: 34 limbs.
+// Two limbs a lane, 2 lane and 2 lane + 1: x += carries of (e[k] at limb k + 1)
+// for the small e, and what runs on; returns the carry out of lane 31.
+__device__ __forceinline__ uint32_t dt_carry2(uint64_t (&x)[2], const uint32_t (&e)[2]) {
+    uint32_t e1 = e[1], in = __shfl_up_sync(0xffffffffu, e1, 1), over;
+    if ((threadIdx.x & 31) == 0) in = 0;
+    x[0] += in;
+    const uint32_t c0 = e[0] + (x[0] < in);
+    x[1] += c0;
+    // what both limbs generate above the lane's own e[1]
+    const uint32_t g = x[1] < c0, cy = dt_lane_carry(g, x[1] == ~0ull && x[0] == ~0ull && !g, over);
+    x[0] += cy;
+    x[1] += (x[0] < cy);
+    return over + __shfl_sync(0xffffffffu, e1, 31);
+}
+
+// The columns of a product, two a lane as above, folded into limbs with
+// `extra` added (dt_fold for two).
+__device__ __forceinline__ uint32_t dt_fold2(const uint64_t (&lo)[2], const uint64_t (&mid)[2], const uint64_t (&hi)[2],
+                                             const uint64_t (&extra)[2], uint64_t (&x)[2]) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint64_t m = __shfl_up_sync(0xffffffffu, mid[1], 1), h0 = __shfl_up_sync(0xffffffffu, hi[0], 1),
+             h1 = __shfl_up_sync(0xffffffffu, hi[1], 1);
+    if (lane == 0) m = h0 = h1 = 0;
+    const uint64_t ms[2] = {m, mid[0]}, hs[2] = {h0, h1};
+    uint32_t e[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        x[k] = lo[k] + ms[k];
+        e[k] = x[k] < ms[k];
+        x[k] += hs[k];
+        e[k] += x[k] < hs[k];
+        x[k] += extra[k];
+        e[k] += x[k] < extra[k];
+    }
+    return dt_carry2(x, e);
+}
+
+// dt_recip's last step for 64 limbs: 32 limbs of y to 64, two columns a lane.
+__device__ __forceinline__ void dt_recip_last(const uint64_t* V, uint64_t* y, uint64_t* t) {
+    constexpr int P = 32;
+    const int lane = (int)(threadIdx.x & 31);
+    const uint64_t* Y = y + P;
+    uint64_t c0[2], c1[2], c2[2], ex[2], S[2];
+    auto column = [&](const uint64_t* X) {
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            c0[k] = c1[k] = 0;
+            uint32_t h = 0;
+            if (2 * lane + k <= P + 1) {
+#pragma unroll 8
+                for (int i = 0; i < P; i++) mac3(c0[k], c1[k], h, X[P - 1 + 2 * lane + k - i], Y[i]);
+            }
+            c2[k] = h;
+        }
+    };
+    // limb j of S and D is column j + 1: index 2 lane + k = j + 1
+    column(V);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = 2 * lane + k;
+        ex[k] = i >= 1 && i <= P + 1 ? V[i - 1] : 0;
+    }
+    dt_fold2(c0, c1, c2, ex, S);
+    const bool pos = (__shfl_sync(0xffffffffu, S[1], (P + 1) / 2) >> 63) == 0;
+    if (!pos) {                    // ~S + 1 from index 1 on
+        uint64_t n0 = lane == 0 ? 0 : ~S[0], n1 = ~S[1];
+        const uint32_t one = lane == 0;
+        n1 += one;
+        uint32_t over;
+        // a lane passes the carry when both its limbs of ~S are all ones
+        const uint32_t g = lane == 0 && n1 == 0, cy = dt_lane_carry(g, lane > 0 && n0 == ~0ull && n1 == ~0ull, over);
+        n0 += cy;
+        n1 += lane > 0 && n0 < cy;
+        S[0] = n0;
+        S[1] = n1;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = 2 * lane + k;
+        if (i >= 1 && i <= P + 1) t[i - 1] = S[k];
+        ex[k] = i >= 1 && i <= P + 1 ? S[k] : 0;
+    }
+    __syncwarp();
+    column(t);
+    uint64_t D[2];
+    dt_fold2(c0, c1, c2, ex, D);
+    // y B^P -+ D: limbs 2 lane, 2 lane + 1 of D are indexes one higher
+    uint64_t d[2] = {D[1], __shfl_down_sync(0xffffffffu, D[0], 1)}, r[2];
+    uint32_t e[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = 2 * lane + k;
+        if (i > P) d[k] = 0;
+        const uint64_t a = i >= P ? Y[i - P] : 0;
+        r[k] = pos ? a - d[k] : a + d[k];
+        e[k] = pos ? a < d[k] : r[k] < d[k];
+    }
+    __syncwarp();
+    uint32_t over;
+    if (pos) {                     // borrows: the same on the complements
+        uint64_t n[2] = {~r[0], ~r[1]};
+        over = dt_carry2(n, e);
+        r[0] = ~n[0];
+        r[1] = ~n[1];
+    } else {
+        over = dt_carry2(r, e);
+    }
+    if (over) r[0] = r[1] = pos ? 0 : ~0ull;
+    y[2 * lane] = r[0];
+    y[2 * lane + 1] = r[1];
+    __syncwarp();
+}
+
+// y[0..LW) = about floor((B^2LW - 1) / V) - B^LW for V = v[0..LW), top bit set,
+// v[LW] = 0, by one warp: Newton's iteration from the top limb's reciprocal,
+// y + 1 = x -> x + x (1 - V x), with 1, 2, .. limbs of y giving twice as many.
+// The top halves of 1 - V x cancel and the lowest columns are left out: within
+// 2^24 (32 limbs) or 2^48 (64) units of the last limb in 3000 random and
+// extreme divisors, which moves a quotient block by one with a chance of 2^-40
+// or 2^-16.  `t`: 66 limbs.
+template <int LW>
 __device__ __forceinline__ void dt_recip(const uint64_t* v, uint64_t* y, uint64_t* t) {
     const int lane = (int)(threadIdx.x & 31);
     t[lane] = 0;
-    if (lane < 2) t[32 + lane] = 0;
-    if (lane == 0) y[31] = recip_limb(v[31]);
+    t[32 + lane] = 0;
+    if (lane < 2) t[64 + lane] = 0;
+    if (lane == 0) y[LW - 1] = recip_limb(v[LW - 1]);
     __syncwarp();
-    dt_recip_step<1>(v, y, t);
-    dt_recip_step<2>(v, y, t);
-    dt_recip_step<4>(v, y, t);
-    dt_recip_step<8>(v, y, t);
-    dt_recip_step<16>(v, y, t);
+    dt_recip_step<1, LW>(v, y, t);
+    dt_recip_step<2, LW>(v, y, t);
+    dt_recip_step<4, LW>(v, y, t);
+    dt_recip_step<8, LW>(v, y, t);
+    dt_recip_step<16, LW>(v, y, t);
+    if constexpr (LW == 64) dt_recip_last(v, y, t);
 }
 
 // One division.  load_u(i) (i < g.MU), load_v(i) (i < g.MV) give limbs,
@@ -224,12 +353,12 @@ __device__ __forceinline__ void dt_recip(const uint64_t* v, uint64_t* y, uint64_
 // results.  `phase` is the barrier's.  Every thread of the CTA calls it and
 // gets the status: 0, 1 for a zero divisor, 2 when the corrections or a wait
 // ran out.
-template <int P, typename LoadU, typename LoadV, typename StoreQ, typename StoreR>
-__device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P>& lay, uint8_t* smem, uint32_t tmem,
+template <int P, int G, typename LoadU, typename LoadV, typename StoreQ, typename StoreR>
+__device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P, G>& lay, uint8_t* smem, uint32_t tmem,
                                              uint32_t& phase, LoadU load_u, LoadV load_v, StoreQ store_q,
                                              StoreR store_r) {
-    using S = DtShape<P>;
-    constexpr int Q = S::Q, H = S::H, NT = S::NT, QT = S::QT;
+    using S = DtShape<P, G>;
+    constexpr int Q = S::Q, H = S::H, NT = S::NT, QT = S::QT, LW = S::LW, KB = S::KB;
     const int tid = (int)threadIdx.x, lane = tid & 31;
     const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     uint64_t* win = reinterpret_cast<uint64_t*>(smem + lay.win);
@@ -258,7 +387,7 @@ __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P>& l
         return 1;
     }
     const int s = __clzll((long long)load_v((uint32_t)K - 1));
-    const int Kp = K < 32 ? 32 : K, z = Kp - K;
+    const int Kp = K < LW ? LW : K, z = Kp - K;
     // limb x of the divisor scaled by 2^s B^z, zero from Kp on
     auto vlimb = [&](int x) -> uint64_t {
         x -= z;
@@ -267,17 +396,20 @@ __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P>& l
         if (s && x > 0) v |= load_v((uint32_t)x - 1) >> (64 - s);
         return v;
     };
-    const int nb = (MU + 1 - K + DT_KB - 1) / DT_KB;
-    const int len = nb * DT_KB + Kp;
+    const int nb = (MU + 1 - K + KB - 1) / KB;
+    const int len = nb * KB + Kp;
     const uint64_t vtop = vlimb(Kp - 1);
 
-    // ---- the reciprocal of the top 32 limbs, on one warp
+    // ---- the reciprocal of the top LW limbs, on one warp
     if (warp == 0) {
-        qh[lane] = vlimb(Kp - 32 + lane);
-        if (lane < 2) qh[32 + lane] = 0;
-        inv[32 + lane] = 0;
+#pragma unroll
+        for (int k = 0; k < G; k++) {
+            qh[32 * k + lane] = vlimb(Kp - LW + 32 * k + lane);
+            inv[LW + 32 * k + lane] = 0;
+        }
+        if (lane < 2) qh[LW + lane] = 0;
         __syncwarp();
-        dt_recip(qh, inv, part);
+        dt_recip<LW>(qh, inv, part);
     } else {
         // the other warps: the window, the dividend scaled by 2^s B^z
         for (int i = tid - 32; i < len; i += NT - 32) {
@@ -290,8 +422,8 @@ __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P>& l
             const int row = i / Q, q = i - row * Q, x = (row + S::KMIN) * Q + q;
             if (x < 0 || x > Kp) *reinterpret_cast<uint4*>(smem + (q * S::R + row) * 16) = make_uint4(0, 0, 0, 0);
         }
-        for (int i = tid - 32 - S::QLO; i < 32 + S::QHI; i += NT - 32)
-            if (i < 0 || i >= 32) qraw[i] = DT_HALF;
+        for (int i = tid - 32 - S::QLO; i < LW + S::QHI; i += NT - 32)
+            if (i < 0 || i >= LW) qraw[i] = DT_HALF;
     }
     // ---- the divisor's balanced digits: Kp + 1 limbs of V + 0x8080..80
     {
@@ -317,51 +449,80 @@ __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P>& l
     bool ok = true;
     int fixes = 0;
     for (int blk = nb - 1; blk >= 0; blk--) {
-        const int w0 = blk * DT_KB;          // the window: limbs w0 .. w0 + Kp + 30
-        // ---- estimate: columns 31 .. 62 of Wt inv, each warp its share of every column
-        {
+        const int w0 = blk * KB;          // the window: limbs w0 .. w0 + Kp + 30
+        // ---- estimate: columns LW - 1 .. 2 LW - 2 of Wt inv, each warp its share of every column
+#pragma unroll
+        for (int k = 0; k < G; k++) {
             uint64_t c0 = 0, c1 = 0;
             uint32_t c2 = 0;
-            const uint64_t* iv = inv + 31 + lane - (int)warp;
+            const uint64_t* iv = inv + LW - 1 + 32 * k + lane - (int)warp;
 #pragma unroll
-            for (int e = 0; e < 1024 / NT; e++) mac3(c0, c1, c2, win[S::at(w0 + Kp - 1 + (int)warp + NT / 32 * e)], iv[-(NT / 32) * e]);
-            part[tid] = c0;
-            part[NT + tid] = c1;
-            part[2 * NT + tid] = c2;
+            for (int e = 0; e < 32 * LW / NT; e++)
+                mac3(c0, c1, c2, win[S::at(w0 + Kp - 1 + (int)warp + NT / 32 * e)], iv[-(NT / 32) * e]);
+            const int at = (int)warp * LW + 32 * k + lane;
+            part[at] = c0;
+            part[G * NT + at] = c1;
+            part[2 * G * NT + at] = c2;
         }
         __syncthreads();
         if (warp == 0) {
-            uint64_t lo = 0, mid = 0, hi = 0;
+            uint64_t lo[G], mid[G], hi[G];
 #pragma unroll
-            for (int e = 0; e < NT / 32; e++) {
-                const uint64_t a = part[32 * e + lane], b = part[NT + 32 * e + lane];
-                lo += a;
-                const uint64_t cb = b + (lo < a);
-                mid += cb;
-                hi += part[2 * NT + 32 * e + lane] + (mid < cb) + (cb < b);
+            for (int k = 0; k < G; k++) {
+                lo[k] = mid[k] = hi[k] = 0;
+#pragma unroll
+                for (int e = 0; e < NT / 32; e++) {
+                    const int at = LW * e + G * lane + k;
+                    const uint64_t a = part[at], b = part[G * NT + at];
+                    lo[k] += a;
+                    const uint64_t cb = b + (lo[k] < a);
+                    mid[k] += cb;
+                    hi[k] += part[2 * G * NT + at] + (mid[k] < cb) + (cb < b);
+                }
             }
-            // limb i: the low part of column 32 + i, the middle of 31 + i, the high of 30 + i, and Wt
-            uint64_t x = __shfl_down_sync(0xffffffffu, lo, 1), y = __shfl_up_sync(0xffffffffu, hi, 1);
-            if (lane == 31) x = 0;
-            if (lane == 0) y = 0;
-            uint64_t sum = x + mid;
-            uint32_t e = sum < x;
-            sum += y;
-            e += sum < y;
-            const uint64_t wl = win[S::at(w0 + Kp - 1 + lane)];
-            sum += wl;
-            e += sum < wl;
-            uint32_t ein = __shfl_up_sync(0xffffffffu, e, 1), over;
-            if (lane == 0) ein = 0;
-            const uint64_t t = sum + ein;
-            const uint64_t fin = t + dt_lane_carry(t < ein, t == ~0ull, over);
-            over += __shfl_sync(0xffffffffu, e, 31);
-            uint64_t qt = __shfl_down_sync(0xffffffffu, fin, 1);
-            if (over) qt = ~0ull;
-            if (lane == 31) qt = 0;
-            qh[lane] = qt;
-            const uint64_t bt = qt + DT_HALF;
-            qraw[lane] = bt + dt_lane_carry(bt < DT_HALF, bt == ~0ull, over);
+            // limb i: the low part of column LW + i, the middle of the one below, the high of the next, and Wt
+            uint64_t below_hi = __shfl_up_sync(0xffffffffu, hi[G - 1], 1), above_lo = __shfl_down_sync(0xffffffffu, lo[0], 1);
+            if (lane == 0) below_hi = 0;
+            if (lane == 31) above_lo = 0;
+            uint64_t sum[G];
+            uint32_t e[G], over;
+#pragma unroll
+            for (int k = 0; k < G; k++) {
+                const uint64_t x = k + 1 < G ? lo[(k + 1) % G] : above_lo, y = k > 0 ? hi[(k + G - 1) % G] : below_hi;
+                sum[k] = x + mid[k];
+                e[k] = sum[k] < x;
+                sum[k] += y;
+                e[k] += sum[k] < y;
+                const uint64_t wl = win[S::at(w0 + Kp - 1 + G * lane + k)];
+                sum[k] += wl;
+                e[k] += sum[k] < wl;
+            }
+            if constexpr (G == 1) {
+                uint32_t ein = __shfl_up_sync(0xffffffffu, e[0], 1);
+                if (lane == 0) ein = 0;
+                sum[0] += ein;
+                sum[0] += dt_lane_carry(sum[0] < ein, sum[0] == ~0ull, over);
+                over += __shfl_sync(0xffffffffu, e[0], 31);
+            } else {
+                over = dt_carry2(sum, e);
+            }
+            // the quotient block is limbs 1 .. : balanced digits of it, and itself
+            uint64_t qt[G], bt[G];
+            qt[G - 1] = __shfl_down_sync(0xffffffffu, sum[0], 1);
+            if constexpr (G == 2) qt[0] = sum[G - 1];
+            uint32_t be[G];
+#pragma unroll
+            for (int k = 0; k < G; k++) {
+                if (over) qt[k] = ~0ull;
+                if (k == G - 1 && lane == 31) qt[k] = 0;
+                qh[G * lane + k] = qt[k];
+                bt[k] = qt[k] + DT_HALF;
+                be[k] = bt[k] < DT_HALF;
+            }
+            if constexpr (G == 1) bt[0] += dt_lane_carry(be[0], bt[0] == ~0ull, over);
+            else dt_carry2(bt, be);
+#pragma unroll
+            for (int k = 0; k < G; k++) qraw[G * lane + k] = bt[k];
         }
         __syncthreads();
         // ---- q^'s core matrices (multc.cuh's, of the balanced digits)
@@ -401,7 +562,7 @@ __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P>& l
         // half.  Segment sg is limbs QT sg ..; its carry out is signed, and made
         // nonnegative for the next segment by 2^30, which that one has taken off.
         const int half = H == 1 ? 0 : (int)(warp >> 2), sg = (tid & 127) * H + (H - 1 - half);
-        const int x0 = QT * sg, lim = Kp + DT_KB;
+        const int x0 = QT * sg, lim = Kp + KB;
         uint64_t d[QT];
         int64_t c = sg == 0 ? 0 : -(1ll << 30);
         const uint32_t tb = tmem + (((warp & 3) * 32) << 16) + half * (P / H);
@@ -409,8 +570,8 @@ __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P>& l
             int64_t u0 = 0, u1 = 0;
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                u0 += (int64_t)(int32_t)(__float_as_uint(v[e] + 12582912.0f) - 0x4B400000u) << (8 * e);
-                u1 += (int64_t)(int32_t)(__float_as_uint(v[4 + e] + 12582912.0f) - 0x4B400000u) << (8 * e);
+                u0 += (int64_t)dt_int<G>(v[e]) << (8 * e);
+                u1 += (int64_t)dt_int<G>(v[4 + e]) << (8 * e);
             }
             const __int128 t = (__int128)(unsigned __int128)(x0 + k < lim ? win[S::at(w0 + x0 + k)] : 0) + c - u0 - ((__int128)u1 << 32);
             d[k] = (uint64_t)t;
@@ -494,7 +655,7 @@ __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P>& l
             }
             if (tid == 0 && step != 0) {          // the quotient block by as much
                 uint64_t k = (uint64_t)(step < 0 ? -step : step);
-                for (int i = 0; i < DT_KB && k; i++) {
+                for (int i = 0; i < KB && k; i++) {
                     const uint64_t x = qh[i];
                     qh[i] = step < 0 ? x - k : x + k;
                     k = step < 0 ? x < k : qh[i] < k;
@@ -502,10 +663,10 @@ __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P>& l
             }
             __syncthreads();
         }
-        if (tid < DT_KB && blk * DT_KB + tid < MU) store_q((uint32_t)(blk * DT_KB + tid), qh[tid]);
+        if (tid < KB && blk * KB + tid < MU) store_q((uint32_t)(blk * KB + tid), qh[tid]);
     }
     // ---- the quotient's zero limbs, the remainder scaled back
-    for (int i = nb * DT_KB + tid; i < MU; i += NT) store_q((uint32_t)i, 0);
+    for (int i = nb * KB + tid; i < MU; i += NT) store_q((uint32_t)i, 0);
     for (int i = tid; i < MV; i += NT) {
         uint64_t x = 0;
         if (i < K) {

@@ -1,4 +1,4 @@
-"""Division in blocks of 31 quotient limbs on the tensor cores against Python
+"""Division in blocks of 31 or 63 quotient limbs on the tensor cores against Python
 integers: both sides of every accumulator width, one to many quotient blocks,
 divisors with leading zero limbs (down to one limb), powers of two, all ones,
 bytes of 0x80 (the largest balanced digits), dividends just below a multiple of
@@ -67,7 +67,8 @@ def _check(B, mu, mv, n, w):
 @pytest.mark.parametrize("mu,mv,n", [
     (64, 40, 12), (130, 65, 12), (129, 66, 700), (200, 130, 24), (446, 223, 24), (447, 224, 24), (512, 256, 320),
     (958, 479, 12), (960, 480, 12), (1470, 735, 12), (1472, 736, 12), (1982, 991, 12), (1984, 992, 12),
-    (2048, 1024, 170), (2494, 1247, 12), (2496, 1248, 12), (4030, 2015, 12), (1055, 1024, 12), (1054, 1024, 12),
+    (2048, 1024, 170), (2430, 1215, 12), (2432, 1216, 12), (2494, 1247, 160), (3966, 1983, 12), (3968, 1984, 12),
+    (4030, 2015, 12), (3000, 1500, 160), (1055, 1024, 12), (1054, 1024, 12),
     (2030, 2010, 12), (8192, 1000, 4), (8192, 2015, 4), (8192, 65, 4)])
 def test_against_integers(bigint, mu, mv, n):
     _check(bigint, mu, mv, n, 64)
