@@ -24,9 +24,12 @@
 // size of the reference's benchmarks), a leaner chunked kernel runs instead:
 // each lane owns 64 consecutive bytes of one instance, so instance
 // boundaries fall only between lanes and the lane's limbs are added or
-// subtracted on the hardware carry chain (chain.cuh).
+// subtracted on the hardware carry chain (chain.cuh).  Differences and 32-bit
+// sums of other sizes, in 16-byte aligned buffers, do the same on chunks that
+// are read from and written to shared memory (the ragged kernel).
 #include "chain.cuh"
 #include "common.cuh"
+#include "multc.cuh"   // mbarrier waits
 
 namespace bi {
 
@@ -517,6 +520,221 @@ addsub_chunk_kernel(const T* a, const T* b, T* r, uint8_t* sign_out, uint32_t cp
 }
 
 // ---------------------------------------------------------------------------
+// Ragged kernel: sizes that are no multiple of 64 bytes, 16-byte aligned
+// buffers.  As the chunked kernel, with chunks of K limbs (K odd) counted from
+// each instance's own start, so that instance boundaries fall between lanes
+// again.  A tile's limbs come to shared memory as they lie (bulk copies of the
+// 16-byte vectors that hold them, the next tile's under way while this one is
+// worked on); the lanes read and write them limb by limb at an odd stride,
+// which meets every bank once, and the tile goes back as vectors, its ends limb
+// by limb.  An instance's last chunk is padded with zeros, which pass a borrow
+// on.  r may be a or b: a tile's limbs are written by its own CTA alone, after
+// they have come.
+//
+// Bound by HBM: 5.8-6.4 TB/s against the row kernel's 3.0 (u32) and 4.5 (u64)
+// for differences, whose two borrow chains a row it resolves limb by limb with
+// ballots.  Chunks of 60 or 56 bytes, as a lane's registers hold both operands
+// twice; 8 warps measured the same as 4 (one barrier set per 14 KB and operand);
+// tiles staged through registers instead of by bulk copies ran at 110-150 us
+// where this takes 66-75 (400 MB), with nothing in flight between barriers.
+// ---------------------------------------------------------------------------
+__device__ uint32_t ragged_gave_up;     // waits for a copy that ran out (never seen)
+
+template <typename T, int W, int K, int OP>
+__global__ void __launch_bounds__(W * 32)
+addsub_ragged_kernel(const T* a, const T* b, T* r, uint8_t* sign_out, uint32_t m, uint32_t cpi, uint64_t n, uint32_t ipt,
+                     uint64_t ntiles) {
+    constexpr int VEC = 16 / sizeof(T);
+    constexpr int NCH = (OP == OP_SUB) ? 2 : 1;
+    constexpr int TILE = W * 32 * K + 2 * VEC;                  // limbs of an operand, with the ends' slack
+    extern __shared__ __align__(16) uint8_t smem_rg[];          // two stages of (a, b)
+    T* stages = reinterpret_cast<T*>(smem_rg);
+    __shared__ uint64_t s_bar[2];
+    __shared__ uint32_t s_gp[NCH][W];   // per-warp composite, bit0 = g, bit1 = p
+    __shared__ uint32_t s_first[W];     // 1 if the warp's first chunk starts an instance
+    __shared__ uint8_t s_sign[(OP == OP_SUB) ? W * 32 : 1];
+
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t q = threadIdx.x / cpi;          // instance within the tile
+    const uint32_t pos = threadIdx.x - q * cpi;    // chunk within the instance
+    const uint32_t rest = m - (pos < cpi - 1 ? pos : cpi - 1) * K;
+    const int cnt = rest < (uint32_t)K ? (int)rest : K;         // the chunk's limbs
+    const uint64_t total = n * m;
+    const uint32_t bars = tc_smem_addr(s_bar);
+    uint64_t once;                      // the operands are read once: first to leave the L2
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(once));
+
+    struct Tile {
+        uint64_t inst0, base;           // first instance; the flat index of its vector's first limb
+        uint32_t ninst;
+        int off, len, bulk;             // limbs before the tile in that vector, of the tile, that a bulk copy brings
+    };
+    auto tile_at = [&](uint64_t tile) {
+        Tile t;
+        t.inst0 = tile * (uint64_t)ipt;
+        const uint64_t left = n - t.inst0, start = t.inst0 * m;
+        t.ninst = left < ipt ? (uint32_t)left : ipt;
+        t.off = (int)(start & (VEC - 1));
+        t.len = (int)(t.ninst * m);
+        t.base = start - t.off;
+        t.bulk = (t.off + t.len + VEC - 1) / VEC * VEC;
+        if (t.base + t.bulk > total) t.bulk = (int)(total - t.base) / VEC * VEC;   // nothing past the buffers
+        return t;
+    };
+    auto fetch = [&](uint64_t tile, int st) {                   // one thread
+        const Tile t = tile_at(tile);
+        const uint32_t bytes = (uint32_t)(t.bulk * sizeof(T)), bar = bars + 8 * st;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * bytes) : "memory");
+        if (bytes == 0) return;
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], "
+                "%4;" ::"r"(tc_smem_addr(stages + (2 * st + k) * TILE)),
+                "l"((k ? b : a) + t.base), "r"(bytes), "r"(bar), "l"(once)
+                : "memory");
+    };
+    if (threadIdx.x == 0) {
+        tc_bar_init(bars, 1);
+        tc_bar_init(bars + 8, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        tc_fence_smem();
+        fetch(blockIdx.x, 0);
+        if (blockIdx.x + (uint64_t)gridDim.x < ntiles) fetch(blockIdx.x + (uint64_t)gridDim.x, 1);
+    }
+    __syncthreads();
+
+    uint32_t it = 0;
+    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
+        const Tile t = tile_at(tile);
+        const int st = (int)(it & 1);
+        T* sx = stages + 2 * st * TILE;
+        T* sy = sx + TILE;
+        const bool valid = q < t.ninst;
+        const bool ok = tc_bar_wait(bars + 8 * st, (it >> 1) & 1);
+        if (__syncthreads_or(!ok)) {
+            if (threadIdx.x == 0) atomicAdd(&ragged_gave_up, 1u);
+            return;
+        }
+        if (t.off + t.len > t.bulk) {                           // the buffers' last limbs
+            const int i = t.bulk + (int)threadIdx.x;
+            if (i < t.off + t.len) {
+                sx[i] = a[t.base + i];
+                sy[i] = b[t.base + i];
+            }
+            __syncthreads();
+        }
+
+        // ---- the lane's chunk
+        T* px = sx + t.off + q * m + pos * K;
+        const T* py = sy + (px - sx);
+        T x[K + 1], y[K + 1];           // and a limb that passes a carry or borrow on
+        x[K] = OP == OP_ADD ? (T)~(T)0 : (T)0;
+        y[K] = 0;
+#pragma unroll
+        for (int e = 0; e < K; e++) {
+            const bool in = valid && e < cnt;
+            x[e] = in ? px[e] : (T)0;
+            y[e] = in ? py[e] : (T)0;
+        }
+        uint32_t g, p;
+        {
+            T c[K + 1];
+#pragma unroll
+            for (int e = 0; e <= K; e++) c[e] = x[e];
+            g = chunk_chain<OP, T, K + 1>(c, y, 0u);
+            T acc = OP == OP_ADD ? (T)~(T)0 : (T)0;
+#pragma unroll
+            for (int e = 0; e < K; e++) {
+                if (OP == OP_ADD) acc &= x[e] ^ y[e];
+                else acc |= x[e] ^ y[e];
+            }
+            p = OP == OP_ADD ? (acc == (T)~(T)0) : (acc == 0);
+            if (!valid) g = p = 0;
+        }
+        const uint32_t S = __ballot_sync(0xffffffffu, valid && pos == 0);
+        const uint32_t kill = S >> 1;   // lane t+1 starts an instance: no carry out of lane t
+        uint32_t A[NCH], B[NCH];
+        A[0] = __ballot_sync(0xffffffffu, g | p) & ~kill;
+        B[0] = __ballot_sync(0xffffffffu, g) & ~kill;
+        if constexpr (OP == OP_SUB) {
+            const uint32_t g2 = (valid && !g && !p) ? 1u : 0u;   // b - a borrows out of this lane
+            A[1] = __ballot_sync(0xffffffffu, g2 | p) & ~kill;
+            B[1] = __ballot_sync(0xffffffffu, g2) & ~kill;
+        }
+        if (lane == 0) {
+#pragma unroll
+            for (int c = 0; c < NCH; c++) {
+                const uint32_t g0 = warp_carry_resolve(A[c], B[c], 0).cout;
+                const uint32_t g1 = warp_carry_resolve(A[c], B[c], 1).cout;
+                s_gp[c][warp] = g0 | ((g1 & ~g0) << 1);
+            }
+            s_first[warp] = S & 1u;
+        }
+        __syncthreads();
+        uint32_t cl[NCH];
+        {
+            const bool before = lane < warp;
+            const bool killed = before && s_first[lane + 1 < W ? lane + 1 : 0];
+#pragma unroll
+            for (int c = 0; c < NCH; c++) {
+                const uint32_t gp = before ? s_gp[c][lane] : 0u;
+                const bool live = before && !killed;
+                const uint32_t A2 = __ballot_sync(0xffffffffu, live && (gp & 3u));
+                const uint32_t B2 = __ballot_sync(0xffffffffu, live && (gp & 1u));
+                uint32_t cin = (warp_carry_resolve(A2, B2, 0).carries >> warp) & 1u;
+                if (S & 1u) cin = 0;
+                cl[c] = (warp_carry_resolve(A[c], B[c], cin).carries >> lane) & 1u;
+            }
+        }
+        if constexpr (OP == OP_SUB) {
+            if (valid && pos == cpi - 1) {
+                const uint8_t sg = (uint8_t)(g | (p & cl[0]));
+                s_sign[q] = sg;
+                if (sign_out) sign_out[t.inst0 + q] = sg;
+            }
+            __syncthreads();
+        }
+        if (valid) {
+            if constexpr (OP == OP_ADD) {
+                chunk_chain<OP_ADD, T, K + 1>(x, y, cl[0]);
+            } else {
+                const bool neg = s_sign[q] != 0;
+                chunk_chain<OP_SUB, T, K + 1>(x, y, neg ? 1u - cl[1] : cl[0]);
+                if (neg) {
+#pragma unroll
+                    for (int e = 0; e < K; e++) x[e] = ~x[e];
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < K; e++)
+                if (e < cnt) px[e] = x[e];
+        }
+        __syncthreads();
+
+        // ---- the tile back
+        const int nvec = (t.off + t.len + VEC - 1) / VEC;
+        for (int v = (int)threadIdx.x; v < nvec; v += W * 32) {
+            const int lo = v * VEC;
+            if (lo >= t.off && lo + VEC <= t.off + t.len) {
+                T o[VEC];
+                *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(sx + lo);
+                store_limbs<T, VEC>(r + t.base + lo, o);
+            } else {
+#pragma unroll
+                for (int e = 0; e < VEC; e++)
+                    if (lo + e >= t.off && lo + e < t.off + t.len) __stcs(r + t.base + lo + e, sx[lo + e]);
+            }
+        }
+        tc_fence_smem();                // this stage's accesses come before the next copy into it
+        __syncthreads();
+        const uint64_t ahead = tile + 2 * (uint64_t)gridDim.x;
+        if (threadIdx.x == 0 && ahead < ntiles) fetch(ahead, st);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Fused add chain, the reference's "ten additions" benchmark
 // (baddKer1Bench, cuda/ker-add.cu.h:88-112; the thesis's 10(u+v),
 // thesis/sections/performance.tex:28-36): r1 = a + b, then p-1 times
@@ -629,6 +847,27 @@ static bi_status launch_chunk(const T* a, const T* b, T* r, uint8_t* sign, uint3
     return launch_chunk_cfg<T, 32, OP>(a, b, r, sign, m, n, st);
 }
 
+template <typename T, int W, int K, int OP>
+static bi_status launch_ragged(const T* a, const T* b, T* r, uint8_t* sign, uint32_t m, uint64_t n, cudaStream_t st) {
+    const uint32_t cpi = (m + K - 1) / K, ipt = (W * 32) / cpi;
+    const uint64_t ntiles = (n + ipt - 1) / ipt;
+    const size_t smem = 4 * (W * 32 * K + 2 * (16 / sizeof(T))) * sizeof(T);
+    auto kern = addsub_ragged_kernel<T, W, K, OP>;
+    cudaError_t e = smem_opt_in((const void*)kern, smem);
+    if (e != cudaSuccess) return set_error(BI_ECUDA, "add/sub: %s", cudaGetErrorString(e));
+    static const int occ = [&] {
+        int o = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, W * 32, smem) != cudaSuccess) {
+            cudaGetLastError();                // not the launch's error: grid one CTA an SM
+            o = 1;
+        }
+        return o > 0 ? o : 1;
+    }();
+    const uint64_t cap = (uint64_t)num_sms() * occ;
+    kern<<<(unsigned)(ntiles < cap ? ntiles : cap), W * 32, smem, st>>>(a, b, r, sign, m, cpi, n, ipt, ntiles);
+    return check_launch(OP == OP_ADD ? "add kernel" : "sub kernel");
+}
+
 // ---------------------------------------------------------------------------
 // Host launch: pick the tile shape for m (the tile must hold one instance).
 // ---------------------------------------------------------------------------
@@ -686,6 +925,20 @@ static bi_status addsub(const T* a, const T* b, T* r, uint8_t* sign, uint32_t m,
     const bool vec16 = ((uintptr_t)a | (uintptr_t)b | (uintptr_t)r) % 16 == 0;
     if (vec16) {
         if (m > max_limbs<T>()) return set_error(BI_EUNSUPPORTED, "m=%u above %u limbs", m, max_limbs<T>());
+        // Odd sizes.  64-bit sums stay with the row kernel, which has them at the
+        // memory rate (235 us for 1.6 GB; ragged 240-270); 32-bit sums and every
+        // difference are bound by its instructions: ragged / row on 1.6 GB, sub
+        // u64 251-276 / 330-362, sub u32 253-295 / 475-854, add u32 240-276 /
+        // 274-495.  Below 5 (u32: 7) limbs most of a lane's chunk would be
+        // padding: sub of 4 u64 limbs 98 / 99 us on 400 MB, of 6 u32 limbs 109 /
+        // 140 but add 87 / 81.
+        if constexpr (OP == OP_SUB || sizeof(T) == 4) {
+            constexpr uint32_t KR = sizeof(T) == 8 ? 7 : 15, LO = sizeof(T) == 8 ? 5 : 7;
+            if (!host_link && m >= LO && m <= 16 * 32 * KR) {
+                if (m <= 8 * 32 * KR) return launch_ragged<T, 8, KR, OP>(a, b, r, sign, m, n, st);
+                return launch_ragged<T, 16, KR, OP>(a, b, r, sign, m, n, st);
+            }
+        }
         return launch_vec<T, 16 / sizeof(T), OP>(a, b, r, sign, m, n, st);
     }
     if (m > max_limbs<T>() / (16 / sizeof(T)))
