@@ -179,6 +179,105 @@ __device__ __forceinline__ uint32_t chain_sub_from(uint64_t (&x)[N], Gen gen, ui
     }
 }
 
+// x[0..2 N - 1] += b (a[0], a[2], .. a[2 N - 2]) as 64-bit products side by side,
+// + c: N wide multiply-adds on the carry flag.  Returns the carry out.
+template <int N>
+__device__ __forceinline__ uint32_t mad_words_n(uint32_t* x, const uint32_t* a, uint32_t b, uint32_t c);
+template <>
+__device__ __forceinline__ uint32_t mad_words_n<1>(uint32_t* x, const uint32_t* a, uint32_t b, uint32_t c) {
+    uint32_t co;
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %5, 0xFFFFFFFF;\n\t"
+        "madc.lo.cc.u32 %0, %3, %4, %0;\n\tmadc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+        "addc.u32 %2, 0, 0;\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "=r"(co)
+        : "r"(a[0]), "r"(b), "r"(c));
+    return co;
+}
+template <>
+__device__ __forceinline__ uint32_t mad_words_n<2>(uint32_t* x, const uint32_t* a, uint32_t b, uint32_t c) {
+    uint32_t co;
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %8, 0xFFFFFFFF;\n\t"
+        "madc.lo.cc.u32 %0, %5, %7, %0;\n\tmadc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+        "madc.lo.cc.u32 %2, %6, %7, %2;\n\tmadc.hi.cc.u32 %3, %6, %7, %3;\n\t"
+        "addc.u32 %4, 0, 0;\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "=r"(co)
+        : "r"(a[0]), "r"(a[2]), "r"(b), "r"(c));
+    return co;
+}
+template <>
+__device__ __forceinline__ uint32_t mad_words_n<4>(uint32_t* x, const uint32_t* a, uint32_t b, uint32_t c) {
+    uint32_t co;
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %14, 0xFFFFFFFF;\n\t"
+        "madc.lo.cc.u32 %0, %9, %13, %0;\n\tmadc.hi.cc.u32 %1, %9, %13, %1;\n\t"
+        "madc.lo.cc.u32 %2, %10, %13, %2;\n\tmadc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+        "madc.lo.cc.u32 %4, %11, %13, %4;\n\tmadc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+        "madc.lo.cc.u32 %6, %12, %13, %6;\n\tmadc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+        "addc.u32 %8, 0, 0;\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]), "=r"(co)
+        : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(a[6]), "r"(b), "r"(c));
+    return co;
+}
+template <>
+__device__ __forceinline__ uint32_t mad_words_n<8>(uint32_t* x, const uint32_t* a, uint32_t b, uint32_t c) {
+    uint32_t co;
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %26, 0xFFFFFFFF;\n\t"
+        "madc.lo.cc.u32 %0, %17, %25, %0;\n\tmadc.hi.cc.u32 %1, %17, %25, %1;\n\t"
+        "madc.lo.cc.u32 %2, %18, %25, %2;\n\tmadc.hi.cc.u32 %3, %18, %25, %3;\n\t"
+        "madc.lo.cc.u32 %4, %19, %25, %4;\n\tmadc.hi.cc.u32 %5, %19, %25, %5;\n\t"
+        "madc.lo.cc.u32 %6, %20, %25, %6;\n\tmadc.hi.cc.u32 %7, %20, %25, %7;\n\t"
+        "madc.lo.cc.u32 %8, %21, %25, %8;\n\tmadc.hi.cc.u32 %9, %21, %25, %9;\n\t"
+        "madc.lo.cc.u32 %10, %22, %25, %10;\n\tmadc.hi.cc.u32 %11, %22, %25, %11;\n\t"
+        "madc.lo.cc.u32 %12, %23, %25, %12;\n\tmadc.hi.cc.u32 %13, %23, %25, %13;\n\t"
+        "madc.lo.cc.u32 %14, %24, %25, %14;\n\tmadc.hi.cc.u32 %15, %24, %25, %15;\n\t"
+        "addc.u32 %16, 0, 0;\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]), "+r"(x[5]), "+r"(x[6]), "+r"(x[7]),
+          "+r"(x[8]), "+r"(x[9]), "+r"(x[10]), "+r"(x[11]), "+r"(x[12]), "+r"(x[13]), "+r"(x[14]), "+r"(x[15]), "=r"(co)
+        : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(a[6]), "r"(a[8]), "r"(a[10]), "r"(a[12]), "r"(a[14]), "r"(b), "r"(c));
+    return co;
+}
+template <int N>
+__device__ __forceinline__ uint32_t mad_words(uint32_t* x, const uint32_t* a, uint32_t b, uint32_t c) {
+    constexpr int Bk = N >= 8 ? 8 : N >= 4 ? 4 : N >= 2 ? 2 : 1;
+    c = mad_words_n<Bk>(x, a, b, c);
+    if constexpr (N > Bk) c = mad_words<N - Bk>(x + 2 * Bk, a + 2 * Bk, b, c);
+    return c;
+}
+
+// x[0..N-1] += y + c over N (even) 32-bit words; returns the carry out.
+template <int N>
+__device__ __forceinline__ uint32_t add_words_n(uint32_t* x, const uint32_t* y, uint32_t c);
+template <>
+__device__ __forceinline__ uint32_t add_words_n<2>(uint32_t* x, const uint32_t* y, uint32_t c) {
+    uint32_t co;
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %5, 0xFFFFFFFF;\n\t"
+        "addc.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\t"
+        "addc.u32 %2, 0, 0;\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "=r"(co)
+        : "r"(y[0]), "r"(y[1]), "r"(c));
+    return co;
+}
+template <>
+__device__ __forceinline__ uint32_t add_words_n<4>(uint32_t* x, const uint32_t* y, uint32_t c) {
+    uint32_t co;
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %9, 0xFFFFFFFF;\n\t"
+        "addc.cc.u32 %0, %0, %5;\n\taddc.cc.u32 %1, %1, %6;\n\taddc.cc.u32 %2, %2, %7;\n\taddc.cc.u32 %3, %3, %8;\n\t"
+        "addc.u32 %4, 0, 0;\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "=r"(co)
+        : "r"(y[0]), "r"(y[1]), "r"(y[2]), "r"(y[3]), "r"(c));
+    return co;
+}
+template <>
+__device__ __forceinline__ uint32_t add_words_n<8>(uint32_t* x, const uint32_t* y, uint32_t c) {
+    return chain_add8(*reinterpret_cast<uint32_t(*)[8]>(x), *reinterpret_cast<const uint32_t(*)[8]>(y), c);
+}
+template <int N>
+__device__ __forceinline__ uint32_t add_words(uint32_t* x, const uint32_t* y, uint32_t c = 0) {
+    constexpr int Bk = N >= 8 ? 8 : N >= 4 ? 4 : 2;
+    c = add_words_n<Bk>(x, y, c);
+    if constexpr (N > Bk) c = add_words<N - Bk>(x + Bk, y + Bk, c);
+    return c;
+}
+
 // The carry out alone (x and y unchanged): the same chain on copies.
 template <typename T>
 __device__ __forceinline__ uint32_t chain_add8_cout(const T (&x)[8], const T (&y)[8], uint32_t c) {

@@ -31,6 +31,8 @@
 // DIV_WARP_MAX_MV, where its K (MU - K + 1) limb products and no barriers
 // cost less than a CTA running the steps above (div_use_long holds the
 // measured crossover, which depends on the batch size too).
+#include <type_traits>
+
 #include "divblock.cuh"
 #include "divtc.cuh"
 #include "divcore.cuh"
@@ -100,11 +102,98 @@ div_thread_kernel(const T* __restrict__ u, const T* __restrict__ v, T* __restric
     }
 }
 
+// The same with the warp's 32 instances in shared memory, a row of SU (SV)
+// 64-bit slots an instance, both odd so that a limb of all lanes meets every
+// bank once.  Rows come and go as consecutive words; the quotient and the
+// remainder take the rows of u and v: quotient limb j is stored after the limbs
+// of u from j up were read, the remainder after all of v was.  Bound by the
+// latency of the carry chains; registers capped for 12 or 14 CTAs an SM (8 to 10
+// as it is, at 8 divisor limbs) made it 4-12 % slower.
+template <typename T>
+__device__ __forceinline__ void rows_in(uint64_t* rows, uint32_t slots, const T* g, uint32_t m, uint32_t count) {
+    constexpr uint32_t PER = 8 / sizeof(T);
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(rows);
+    const uint32_t dr = 32 / m, dc = 32 - dr * m;
+    uint32_t row = (threadIdx.x & 31) / m, col = (threadIdx.x & 31) - row * m;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x & 31; i < count * m; i += 32) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                         base + (row * slots * PER + col) * (uint32_t)sizeof(T)),
+                     "l"(g + i), "n"(sizeof(T))
+                     : "memory");
+        row += dr, col += dc;
+        if (col >= m) col -= m, row++;
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ void rows_out(const uint64_t* rows, uint32_t slots, T* g, uint32_t m, uint32_t count) {
+    constexpr uint32_t PER = 8 / sizeof(T);
+    const T* words = reinterpret_cast<const T*>(rows);
+    const uint32_t dr = 32 / m, dc = 32 - dr * m;
+    uint32_t row = (threadIdx.x & 31) / m, col = (threadIdx.x & 31) - row * m;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x & 31; i < count * m; i += 32) {
+        g[i] = words[row * slots * PER + col];
+        row += dr, col += dc;
+        if (col >= m) col -= m, row++;
+    }
+}
+
+template <typename T, int MX>
+__global__ void __launch_bounds__(DIV_THREAD_CTA)
+div_thread_rows_kernel(const T* __restrict__ u, const T* __restrict__ v, T* __restrict__ q, T* __restrict__ r,
+                       uint8_t* __restrict__ status, uint64_t n, uint32_t mu, uint32_t mv) {
+    extern __shared__ __align__(16) uint64_t smem[];
+    const uint32_t MU = sizeof(T) == 8 ? mu : (mu + 1) / 2, MV = sizeof(T) == 8 ? mv : (mv + 1) / 2;
+    const uint32_t SU = MU | 1, SV = MV | 1, lane = threadIdx.x & 31;
+    uint64_t* ru = smem + threadIdx.x / 32 * 32 * (SU + SV);
+    uint64_t* rv = ru + 32 * SU;
+    uint64_t* mu_row = ru + lane * SU;
+    uint64_t* mv_row = rv + lane * SV;
+    for (uint64_t first = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32 * 32; first < n;
+         first += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t count = n - first < 32 ? (uint32_t)(n - first) : 32u;
+        rows_in(ru, SU, u + first * mu, mu, count);
+        rows_in(rv, SV, v + first * mv, mv, count);
+        if (sizeof(T) == 4 && (mu & 1)) reinterpret_cast<T*>(mu_row)[mu] = 0;   // an odd count's upper word
+        if (sizeof(T) == 4 && (mv & 1)) reinterpret_cast<T*>(mv_row)[mv] = 0;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        if (lane < count) {
+            const uint8_t st = div_thread<MX>(
+                MU, MV, [&](uint32_t i) { return mu_row[i]; }, [&](uint32_t i) { return mv_row[i]; },
+                [&](uint32_t i, uint64_t x) { mu_row[i] = x; }, [&](uint32_t i, uint64_t x) { mv_row[i] = x; });
+            if (status) status[first + lane] = st;
+        }
+        __syncwarp();
+        rows_out(ru, SU, q + first * mu, mu, count);
+        rows_out(rv, SV, r + first * mv, mv, count);
+        __syncwarp();
+    }
+}
+
 // Several instances a warp: long division on G-lane groups (divsmall.cuh).
 template <typename T, int VPL, int G>
 __global__ void __launch_bounds__(DIV_WARP_CTA)
 div_group_kernel(const T* __restrict__ u, const T* __restrict__ v, T* __restrict__ q, T* __restrict__ r,
                  uint8_t* __restrict__ status, uint64_t n, uint32_t mu, uint32_t mv);
+
+// Rows through shared memory, or each thread its own from global memory (us,
+// direct / rows, 1.0e8 bytes of operands unless n is given).  Words of u32 are
+// strided worst: 125 / 72 for 16 by 8 64-bit limbs, 85 / 67 for 8 by 4, but
+// 58 / 69 for 6 by 3.  u64: 72 / 63 for 16 by 8, 92 / 78 for 32 by 16, 64 / 68
+// for 15 by 7, 54 / 61 for 8 by 4.  Batches that do not fill the SMs have rows
+// at less latency: 50000 of 16 by 8 26.8 / 21.3, of 4 by 2 20.7 / 16.0.  Longer
+// rows leave too few warps an SM: u64 64 by 16 124 / 126 and 80 by 15 138 / 150,
+// u32 80 by 15 178 / 162.
+constexpr int DIV_ROWS_PER_SM = 384;
+template <typename T>
+static bool div_thread_rows(uint32_t MU, uint32_t MV, uint64_t n, int sms) {
+    if (sizeof(T) == 4 && MV >= 4) return MU + MV <= 94;
+    if (n <= (uint64_t)DIV_ROWS_PER_SM * (uint64_t)sms) return MU + MV <= 72;
+    return sizeof(T) == 8 && MV >= 8 && MU <= 48;
+}
 
 template <typename T>
 static void launch_div_thread(const T* u, const T* v, T* q, T* r, uint8_t* status, uint32_t mu, uint32_t mv,
@@ -117,16 +206,25 @@ static void launch_div_thread(const T* u, const T* v, T* q, T* r, uint8_t* statu
     }
     const uint64_t blocks = (n + DIV_THREAD_CTA - 1) / DIV_THREAD_CTA;
     const unsigned grid = (unsigned)(blocks < (1u << 20) ? blocks : (1u << 20));
+    const uint32_t MU = sizeof(T) == 8 ? mu : (mu + 1) / 2;
+    const size_t rows = DIV_THREAD_CTA * ((MU | 1) + (MV | 1)) * sizeof(uint64_t);
     // register windows of 2, 3, 4, 6, 8, 12 or 16 limbs: a divisor is
     // right-aligned in its window, whose rows below it are zeros, so the widths
     // between the powers of two ran 6-20 % faster at 3, 5, 6, 10, 12 limbs
-    if (MV <= 2) div_thread_kernel<T, 2><<<grid, DIV_THREAD_CTA, 0, s>>>(u, v, q, r, status, n, mu, mv);
-    else if (MV <= 3) div_thread_kernel<T, 3><<<grid, DIV_THREAD_CTA, 0, s>>>(u, v, q, r, status, n, mu, mv);
-    else if (MV <= 4) div_thread_kernel<T, 4><<<grid, DIV_THREAD_CTA, 0, s>>>(u, v, q, r, status, n, mu, mv);
-    else if (MV <= 6) div_thread_kernel<T, 6><<<grid, DIV_THREAD_CTA, 0, s>>>(u, v, q, r, status, n, mu, mv);
-    else if (MV <= 8) div_thread_kernel<T, 8><<<grid, DIV_THREAD_CTA, 0, s>>>(u, v, q, r, status, n, mu, mv);
-    else if (MV <= 12) div_thread_kernel<T, 12><<<grid, DIV_THREAD_CTA, 0, s>>>(u, v, q, r, status, n, mu, mv);
-    else div_thread_kernel<T, 16><<<grid, DIV_THREAD_CTA, 0, s>>>(u, v, q, r, status, n, mu, mv);
+    auto launch = [&](auto width) {
+        constexpr int MX = decltype(width)::value;
+        if (div_thread_rows<T>(MU, MV, n, num_sms()))   // at most 48 KB of rows
+            div_thread_rows_kernel<T, MX><<<grid, DIV_THREAD_CTA, rows, s>>>(u, v, q, r, status, n, mu, mv);
+        else
+            div_thread_kernel<T, MX><<<grid, DIV_THREAD_CTA, 0, s>>>(u, v, q, r, status, n, mu, mv);
+    };
+    if (MV <= 2) launch(std::integral_constant<int, 2>{});
+    else if (MV <= 3) launch(std::integral_constant<int, 3>{});
+    else if (MV <= 4) launch(std::integral_constant<int, 4>{});
+    else if (MV <= 6) launch(std::integral_constant<int, 6>{});
+    else if (MV <= 8) launch(std::integral_constant<int, 8>{});
+    else if (MV <= 12) launch(std::integral_constant<int, 12>{});
+    else launch(std::integral_constant<int, 16>{});
 }
 
 // One warp per instance: long division for divisors of at most 32 VPL limbs

@@ -129,34 +129,53 @@ __device__ __forceinline__ uint8_t div_thread(uint32_t MU, uint32_t MV, LoadU lo
     }
     const uint64_t d1 = D[MX - 1], d2 = D[MX - 2];
     const uint64_t v3 = recip_3by2(d1, d2, recip_limb(d1));
+    // B^MX - D as 32-bit words: R - q-hat D = R + q-hat N - q-hat B^MX, a sum of
+    // wide multiply-adds on the carry flag: four a limb and two additions, where
+    // high and low products and two borrow chains took about three times the
+    // instructions (32 by 16 limbs 94 -> 92 us, 12 by 6 60 -> 55, 8 by 4 59 -> 54,
+    // 1.0e8 bytes of operands)
+    uint32_t N[2 * MX];
+    {
+        uint64_t c = 1;
+#pragma unroll
+        for (int k = 0; k < MX; k++) {
+            const uint64_t x = ~D[k] + c;
+            c &= x == 0;
+            N[2 * k] = (uint32_t)x;
+            N[2 * k + 1] = (uint32_t)(x >> 32);
+        }
+    }
     int tn = (int)MU - MX - 1;   // shifted-dividend limb that enters the window next
     for (int j = (int)MU - K; j >= 0; j--) {
         // the raw limb this step's slide needs, loaded first so that its
         // latency overlaps the step's arithmetic
         const uint64_t lower = j > 0 ? raw(tn - 1) : 0;
-        const uint64_t u2 = R[MX], u1 = R[MX - 1], u0 = R[MX - 2];
-        uint64_t qh = qhat_3by2(u2, u1, u0, d1, d2, v3);
-        // R -= q-hat * D on the carry flag: the high halves one limb up (R[1..MX]),
-        // then the low halves (R[0..MX-1], the borrow out taken from R[MX]);
-        // the result is negative iff one of the two wrapped
-        const uint32_t bA = chain_sub_from<MX>(*reinterpret_cast<uint64_t(*)[MX]>(&R[1]),
-                                               [&](int k) { return __umul64hi(qh, D[k]); }, 0);
-        const uint32_t bo = chain_sub_from<MX>(*reinterpret_cast<uint64_t(*)[MX]>(&R[0]),
-                                               [&](int k) { return qh * D[k]; }, 0);
-        const bool bB = R[MX] < bo;
-        R[MX] -= bo;
-        const bool borrow = bA != 0 || bB;
-        if (borrow) {                          // one too large after all: add D back
-            qh -= 1;
-            uint64_t c = 0;
+        uint64_t qh = qhat_3by2(R[MX], R[MX - 1], R[MX - 2], d1, d2, v3);
+        const uint32_t q0 = (uint32_t)qh, q1 = (uint32_t)(qh >> 32);
+        uint32_t W[2 * MX + 2], O[2 * MX + 1];   // the window's words; products that start at an odd word
 #pragma unroll
-            for (int k = 0; k < MX; k++) {
-                const uint64_t x = R[k] + D[k];
-                const uint64_t c1 = x < D[k] ? 1 : 0;
-                R[k] = x + c;
-                c = c1 | (R[k] < x ? 1 : 0);
-            }
-            R[MX] += c;
+        for (int k = 0; k <= MX; k++) {
+            W[2 * k] = (uint32_t)R[k];
+            W[2 * k + 1] = (uint32_t)(R[k] >> 32);
+        }
+#pragma unroll
+        for (int k = 0; k < MX; k++) {
+            const uint64_t x = (uint64_t)N[2 * k + 1] * q0;
+            O[2 * k] = (uint32_t)x;
+            O[2 * k + 1] = (uint32_t)(x >> 32);
+        }
+        O[2 * MX] = mad_words<MX>(O, N, q1, 0);
+        const uint32_t c0 = mad_words<MX>(W, N, q0, 0);
+        mad_words<MX>(W + 2, N + 1, q1, 0);
+        const uint32_t c1 = add_words<2 * MX>(W + 1, O);
+#pragma unroll
+        for (int k = 0; k < MX; k++) R[k] = ((uint64_t)W[2 * k + 1] << 32) | W[2 * k];
+        uint64_t top = ((uint64_t)(W[2 * MX + 1] + O[2 * MX] + c1) << 32) | W[2 * MX];
+        top += c0;
+        top -= qh;
+        if (top != 0) {                        // -1: q-hat was one too large after all, add D back
+            qh -= 1;
+            chain_sub_gen<MX>(&R[0], [&](int k) { return ((uint64_t)N[2 * k + 1] << 32) | N[2 * k]; }, 0);
         }
         store_q((uint32_t)j, qh);
         if (j > 0) {                           // slide the window down one limb
