@@ -30,7 +30,9 @@
 // DIV_THREAD_MAX_MV 64-bit limbs and on one warp per instance up to
 // DIV_WARP_MAX_MV, where its K (MU - K + 1) limb products and no barriers
 // cost less than a CTA running the steps above (div_use_long holds the
-// measured crossover, which depends on the batch size too).
+// measured crossover, which depends on the batch size too).  Medium and large
+// divisors go by blocks of quotient limbs to the tensor cores (divtc.cuh) where
+// div_use_tc says so, and the two routes above keep the rest.
 #include <type_traits>
 
 #include "divblock.cuh"
