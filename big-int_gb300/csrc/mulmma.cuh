@@ -15,7 +15,8 @@
 //
 // Digits are balanced, in [-128, 127]: byte k of x + 0x8080..80 less 128, and
 // one more digit, the carry.  A sum of 1024 products of at most 2^14 is an
-// exact f32; above 128 limbs the sums move to integers halfway.
+// exact f32; above 128 limbs the sums move to integers halfway, after residues
+// 0 .. 3: at 256 limbs (2048 products in the last column) both halves are 1024.
 //
 // Bound by the tensor core's legacy rate (8 cycles an instruction and a quarter
 // SM: 338 cycles an instance of 64 limbs) and the instructions around it (229),
@@ -189,6 +190,15 @@ __device__ __forceinline__ void mm_product(const Item& it, const MmLimbs<MmShape
     // ldmatrix: rows lane & 7 of the four 8 x 8 parts (rows 0.., rows 8.., then the same 8 digits on)
     const uint32_t ap = (uint32_t)__cvta_generic_to_shared(a16) +
                         16 * ((lane & 7) + ((lane >> 3) & 1) * 8) + 16 * (lane >> 4);
+    {   // r = 0, w = 0: before the move below, so that both halves hold at most 1024 products a column
+        const uint32_t b0 = bp[0], b1 = bp[-4];
+#pragma unroll
+        for (int v = 0; v < (FULL ? LT + 1 : LT); v++) {
+            uint32_t a[4];
+            mm_ldmatrix(a, ap + 256 * v);
+            mm_mma(c[v], a, b0, b1);
+        }
+    }
     // (all residues unrolled run 8-10 % faster up to 64 limbs, slower above)
 #pragma unroll (LT <= 5 ? 8 : 1)
     for (int r = 0; r < 8; r++) {
@@ -220,15 +230,6 @@ __device__ __forceinline__ void mm_product(const Item& it, const MmLimbs<MmShape
                     ci[u][k] = __float2int_rn(c[u][k]);
                     c[u][k] = 0;
                 }
-        }
-    }
-    {   // r = 0, w = 0
-        const uint32_t b0 = bp[0], b1 = bp[-4];
-#pragma unroll
-        for (int v = 0; v < (FULL ? LT + 1 : LT); v++) {
-            uint32_t a[4];
-            mm_ldmatrix(a, ap + 256 * v);
-            mm_mma(c[v], a, b0, b1);
         }
     }
     __syncwarp();   // the operands are read
