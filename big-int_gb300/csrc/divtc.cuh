@@ -12,8 +12,9 @@
 //   subtract  each thread folds its accumulator row with its window limbs, one
 //             carry lookahead joins the rows;
 //   check     a negative window or one not below the divisor (q^ is at most
-//             one too large, two too small; both take chance 2^-58 or so on
-//             random operands) is corrected with the whole CTA.
+//             one too large or too small; on random operands with a chance of
+//             about 2^-40 at 32 limbs, 2^-16 at 64) is corrected with the whole
+//             CTA.
 // Digits are balanced, in [-128, 127]: byte k of x + 0x8080..80 less 128.  A
 // column then sums at most 249 or 505 products (q^ has LW - 1 limbs and a carry
 // digit) of magnitude 2^14 at most, below 2^22 or 2^23: one accumulator holds a
@@ -22,11 +23,14 @@
 // pay for it with a longer reciprocal and four times the estimate's products.
 //
 // With W < V B^(LW-1), V's top bit set and K >= LW limbs, Wt and Vh the top LW
-// limbs of W (K + LW - 1 limbs) and V and I = floor((B^2LW - 1) / Vh): q^ =
-// floor((floor(Wt (I - B^LW) / B^LW) + Wt) / B) differs from floor(W / V) by at
-// most one either way, and by one more below for the columns of the product
-// that are left out.  A divisor of fewer than LW limbs is scaled by B^(LW-K),
-// which scales the remainder.
+// limbs of W (K + LW - 1 limbs) and V and I the reciprocal floor((B^2LW - 1) / Vh):
+// q^ = floor((floor(Wt (I - B^LW) / B^LW) + Wt) / B).  Against W / V the limbs
+// below Vh and Wt, the roundings and the columns of the product that are left out
+// weigh less than LW + 8 units of the limb that the last division by B takes off,
+// and the error of I (dt_recip: below 2^29 or 2^57) at most as many: together far
+// below one, so that q^ differs from floor(W / V) by at most one either way.  A
+// divisor of fewer than LW limbs is scaled by B^(LW-K), which scales the
+// remainder.
 #pragma once
 
 #include "divsmall.cuh"
@@ -36,7 +40,7 @@
 namespace bi {
 
 constexpr uint64_t DT_HALF = 0x8080808080808080ull;
-constexpr int DT_MAX_CORRECTIONS = 4;
+constexpr int DT_MAX_CORRECTIONS = 4;    // one is needed at most
 
 // G: limbs a lane of LW = 32 G
 template <int P, int G>
@@ -326,19 +330,27 @@ __device__ __forceinline__ void dt_recip_last(const uint64_t* V, uint64_t* y, ui
 }
 
 // y[0..LW) = about floor((B^2LW - 1) / V) - B^LW for V = v[0..LW), top bit set,
-// v[LW] = 0, by one warp: Newton's iteration from the top limb's reciprocal,
-// y + 1 = x -> x + x (1 - V x), with 1, 2, .. limbs of y giving twice as many.
-// The top halves of 1 - V x cancel and the lowest columns are left out: within
-// 2^24 (32 limbs) or 2^48 (64) units of the last limb in 3000 random and
-// extreme divisors, which moves a quotient block by one with a chance of 2^-40
-// or 2^-16.  `t`: 66 limbs.
+// v[LW] = 0, by one warp: Newton's iteration x -> x + x (1 - V x) on x = 1 + y
+// (V in [1/2, 1), y a fraction), from the reciprocal of the top two limbs, with
+// 1, 2, .. limbs of y giving twice as many.
+//
+// Error: let eta = (1 - V x) B^P at P limbs.  A step leaves out less than P + 2
+// units of the residual (P of columns, 2 of V's limbs below) and less than P of
+// the correction, so that eta' lies above -(P + 2), or -(2 P + 2) where eta is
+// negative, and below max eta^2 + P.  The two-limb start has eta in [0, 1) but
+// for 2 / B, which gives (-3, 2), (-6, 11), (-10, 125), (-18, 15633), then below
+// 2^28 at 32 limbs and 2^56 at 64; y is off by at most 2 eta + 1 of its last
+// unit, 2^29 or 2^57.  Random divisors have some 2^24 and 2^48.  (A one-limb
+// start has eta up to 2, and 2^34 and 2^66 where the top limb is just above 2^63
+// and the next all ones: there nine quotient blocks of ten were one or two short
+// at 64 limbs.)  `t`: 66 limbs.
 template <int LW>
 __device__ __forceinline__ void dt_recip(const uint64_t* v, uint64_t* y, uint64_t* t) {
     const int lane = (int)(threadIdx.x & 31);
     t[lane] = 0;
     t[32 + lane] = 0;
     if (lane < 2) t[64 + lane] = 0;
-    if (lane == 0) y[LW - 1] = recip_limb(v[LW - 1]);
+    if (lane == 0) y[LW - 1] = recip_3by2(v[LW - 1], v[LW - 2], recip_limb(v[LW - 1]));
     __syncwarp();
     dt_recip_step<1, LW>(v, y, t);
     dt_recip_step<2, LW>(v, y, t);
