@@ -82,6 +82,7 @@ SIGNATURES: dict[str, list] = {
     "bi_status_string": [_I],
     "bi_last_error": [],
     "bi_version": [],
+    "bi_wait_status": [_I],
     "bi_max_limbs_addsub_u64": [],
     "bi_max_limbs_addsub_u32": [],
     "bi_fill_splitmix64": [_P, _U64, _U64, _U64, _P],
@@ -120,6 +121,7 @@ SIGNATURES: dict[str, list] = {
     "bi_batch_noalloc_max_descs": [],
     "bi_batch_run_noalloc": [_P, _U64, _P, _U64, _P, _U64, _P, _U64, _P],
     "bi_probe_intpipe": [_P, _P],
+    "bi_probe_held_wait": [_I, _P, _P, _P, _P, _U32, _U64, _P],
     "bi_add_chain_u64": [_P, _P, _P, _U32, _U64, _U32, _P],
     "bi_add_chain_u32": [_P, _P, _P, _U32, _U64, _U32, _P],
     "bi_mul_chain_u64": [_P, _P, _P, _U32, _U64, _U32, _P],
@@ -178,6 +180,13 @@ def _check(status: int) -> None:
     if status != 0:
         detail = lib().bi_last_error().decode(errors="replace")
         raise BigIntError(status, detail)
+
+
+def wait_status(clear: bool = False) -> int:
+    """0, or 4 (BI_ETIMEDOUT) if a device-side wait of a finished kernel ran
+    out on the current device: results since then are incomplete, and every
+    call raises until it is cleared here."""
+    return lib().bi_wait_status(1 if clear else 0)
 
 
 # ---------------------------------------------------------------------------

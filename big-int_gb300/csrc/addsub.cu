@@ -538,12 +538,10 @@ addsub_chunk_kernel(const T* a, const T* b, T* r, uint8_t* sign_out, uint32_t cp
 // tiles staged through registers instead of by bulk copies ran at 110-150 us
 // where this takes 66-75 (400 MB), with nothing in flight between barriers.
 // ---------------------------------------------------------------------------
-__device__ uint32_t ragged_gave_up;     // waits for a copy that ran out (never seen)
-
 template <typename T, int W, int K, int OP>
 __global__ void __launch_bounds__(W * 32)
 addsub_ragged_kernel(const T* a, const T* b, T* r, uint8_t* sign_out, uint32_t m, uint32_t cpi, uint64_t n, uint32_t ipt,
-                     uint64_t ntiles) {
+                     uint64_t ntiles, uint32_t* gave_up) {
     constexpr int VEC = 16 / sizeof(T);
     constexpr int NCH = (OP == OP_SUB) ? 2 : 1;
     constexpr int TILE = W * 32 * K + 2 * VEC;                  // limbs of an operand, with the ends' slack
@@ -614,7 +612,7 @@ addsub_ragged_kernel(const T* a, const T* b, T* r, uint8_t* sign_out, uint32_t m
         const bool valid = q < t.ninst;
         const bool ok = tc_bar_wait(bars + 8 * st, (it >> 1) & 1);
         if (__syncthreads_or(!ok)) {
-            if (threadIdx.x == 0) atomicAdd(&ragged_gave_up, 1u);
+            if (threadIdx.x == 0) report_gave_up(gave_up);
             return;
         }
         if (t.off + t.len > t.bulk) {                           // the buffers' last limbs
@@ -863,8 +861,10 @@ static bi_status launch_ragged(const T* a, const T* b, T* r, uint8_t* sign, uint
         }
         return o > 0 ? o : 1;
     }();
+    uint32_t* gave_up;
+    BI_RETURN_IF(gave_up_word(&gave_up));
     const uint64_t cap = (uint64_t)num_sms() * occ;
-    kern<<<(unsigned)(ntiles < cap ? ntiles : cap), W * 32, smem, st>>>(a, b, r, sign, m, cpi, n, ipt, ntiles);
+    kern<<<(unsigned)(ntiles < cap ? ntiles : cap), W * 32, smem, st>>>(a, b, r, sign, m, cpi, n, ipt, ntiles, gave_up);
     return check_launch(OP == OP_ADD ? "add kernel" : "sub kernel");
 }
 
@@ -917,6 +917,7 @@ static bi_status addsub(const T* a, const T* b, T* r, uint8_t* sign, uint32_t m,
         return set_error(BI_EINVAL, "buffers must be aligned to the limb size");
     if ((uint64_t)n * m / m != n || n * (uint64_t)m > (1ull << 46))
         return set_error(BI_EINVAL, "n*m too large");
+    BI_RETURN_IF(waits_ok());
     cudaStream_t st = (cudaStream_t)s;
     const bool vec32 = ((uintptr_t)a | (uintptr_t)b | (uintptr_t)r) % 32 == 0;
     constexpr uint32_t KC = 64 / sizeof(T);
@@ -958,6 +959,7 @@ static bi_status add_chain(const T* a, const T* b, T* r, uint32_t m, uint64_t n,
     if ((uintptr_t)a % sizeof(T) || (uintptr_t)b % sizeof(T) || (uintptr_t)r % sizeof(T))
         return set_error(BI_EINVAL, "buffers must be aligned to the limb size");
     if ((uint64_t)n * m > (1ull << 46)) return set_error(BI_EINVAL, "n*m too large");
+    BI_RETURN_IF(waits_ok());
     constexpr uint32_t KC = 64 / sizeof(T);
     cudaStream_t st = (cudaStream_t)s;
     if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)r) % 32 == 0 && m % KC == 0 && m <= 32 * 32 * KC) {

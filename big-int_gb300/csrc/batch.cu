@@ -277,14 +277,12 @@ struct TcItem {                        // an instance of the batch
     __device__ __forceinline__ void store(uint32_t x, uint64_t v) const { st64(out, orr, outm, w32, x, v); }
 };
 
-__device__ uint32_t batch_tc_gave_up;    // waits on the tensor core that ran out (never seen)
-
 template <int P>
 __global__ void __launch_bounds__(TcShape<P>::THREADS, 1)
 batch_multc_kernel(const bi_desc* __restrict__ descs, const uint32_t* __restrict__ list, uint32_t count,
-                   const uint64_t* in, uint64_t* out, TcGeom g) {
+                   const uint64_t* in, uint64_t* out, TcGeom g, uint32_t* gave_up) {
     extern __shared__ __align__(128) uint8_t smem_tc[];
-    tc_products<P>(g, smem_tc, blockIdx.x, gridDim.x, count, &batch_tc_gave_up, [&](uint64_t i) {
+    tc_products<P>(g, smem_tc, blockIdx.x, gridDim.x, count, gave_up, [&](uint64_t i) {
         const bi_desc& d = descs[list[i]];
         const uint32_t m = d.m, outm = d.op == BI_OP_MULFULL ? 2 * m : m;
         const bool w32 = desc_w32(d);
@@ -775,6 +773,8 @@ static bi_status launch_plan_kernels(bi_plan* p, const uint64_t* in, uint64_t* o
             batch_addsub_kernel<1, 4><<<grid, 256, 0, s_add>>>(p->d_descs, p->d_addsub, p->n_addsub, p->d_counters + 0, in, out, flags);
         BI_RETURN_IF(check_launch("batch add/sub kernel"));
     }
+    uint32_t* gave_up;
+    BI_RETURN_IF(gave_up_word(&gave_up));
     if (comps & COMP_MUL) {
         const bool small_warp = plan_small_on_warps(p, t);
         const MulItem* items = small_warp ? p->d_items_large : p->d_items;
@@ -807,7 +807,7 @@ static bi_status launch_plan_kernels(bi_plan* p, const uint64_t* in, uint64_t* o
             size_t smem = 0;
             const void* k = multc_class_kernel(c, p->multc_geom[c], &threads, &cols, &smem);
             const uint32_t* list = p->d_multc + p->multc_off[c];
-            void* args[] = {&p->d_descs, &list, &n, &in, &out, &p->multc_geom[c]};
+            void* args[] = {&p->d_descs, &list, &n, &in, &out, &p->multc_geom[c], &gave_up};
             cudaLaunchKernel(k, dim3(L.grid[PLAN_MULTC0 + c]), dim3(threads), args, smem, s[PLAN_MULTC0 + c]);
             BI_RETURN_IF(check_launch("batch tensor mul kernel"));
         }
@@ -1142,6 +1142,7 @@ bi_status bi_plan_execute(bi_plan* p, const uint64_t* in, uint64_t* out, uint8_t
     if (!in || !out) return set_error(BI_EINVAL, "NULL arena");
     if (flags && p->nflags == 0) return set_error(BI_EINVAL, "flags given to a plan created with nflags = 0");
     if ((uintptr_t)in % 16 || (uintptr_t)out % 16) return set_error(BI_EINVAL, "arenas must be 16-byte aligned");
+    BI_RETURN_IF(waits_ok());
     std::lock_guard<std::mutex> lk(p->mu);
     if (!p->exec || p->g_in != in || p->g_out != out || p->g_flags != flags ||
         memcmp(&p->g_tune, &p->tune, sizeof(BatchTune)) != 0) {
@@ -1200,6 +1201,7 @@ bi_status bi_plan_autotune(bi_plan* p, const uint64_t* in, uint64_t* out, uint8_
     if (!in || !out) return set_error(BI_EINVAL, "NULL arena");
     if (flags && p->nflags == 0) return set_error(BI_EINVAL, "flags given to a plan created with nflags = 0");
     if (reps < 1) reps = 1;
+    BI_RETURN_IF(waits_ok());
     std::lock_guard<std::mutex> lk(p->mu);
     BatchTune best = p->tune;
     if (p->n_addsub) {
@@ -1234,6 +1236,7 @@ bi_status bi_plan_autotune(bi_plan* p, const uint64_t* in, uint64_t* out, uint8_
     }
     cudaError_t e = cudaStreamSynchronize(p->cap);
     if (e != cudaSuccess) return set_error(BI_ECUDA, "autotune: %s", cudaGetErrorString(e));
+    BI_RETURN_IF(waits_ok());
     p->tune = best;
     if (chosen) {
         chosen[0] = best.addsub_rows;
@@ -1339,6 +1342,7 @@ extern "C" bi_status bi_batch_run_noalloc(const bi_desc* descs, uint64_t count, 
     }
     if (cs != cudaStreamCaptureStatusNone)
         return set_error(BI_EUNSUPPORTED, "bi_batch_run_noalloc: the stream is being captured");
+    BI_RETURN_IF(waits_ok());
     std::lock_guard<std::mutex> lk(na_mu);
     void* scratch = nullptr;
     BI_RETURN_IF(noalloc_scratch(&scratch));
@@ -1422,5 +1426,5 @@ extern "C" bi_status bi_batch_run_noalloc(const bi_desc* descs, uint64_t count, 
     // the host staging arrays may be reused once the copies have read them
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return set_error(BI_ECUDA, "batch run: %s", cudaGetErrorString(e));
-    return BI_OK;
+    return waits_ok();
 }

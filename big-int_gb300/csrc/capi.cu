@@ -73,6 +73,52 @@ cudaError_t smem_opt_in(const void* func, size_t smem) {
     return e;
 }
 
+// A line of host memory a device, written by a kernel whose wait ran out and read
+// by every later call: no copy, no synchronisation, and the results that are
+// missing are reported whoever asks next.  Static, so that the host may read it
+// whatever became of the CUDA context; the device address is looked up on every
+// call, so that a context that was created anew registers it anew.
+alignas(4096) static uint32_t g_gave_up[64][16];
+
+static int gave_up_line() {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess ? dev & 63 : -1;
+}
+
+bi_status gave_up_word(uint32_t** word) {
+    void* base = nullptr;
+    const int line = gave_up_line();
+    cudaError_t e = line < 0 ? cudaGetLastError() : cudaHostGetDevicePointer(&base, g_gave_up, 0);
+    if (line >= 0 && e != cudaSuccess) {
+        cudaGetLastError();
+        static std::mutex mu;
+        std::lock_guard<std::mutex> lk(mu);
+        // no stream operation, so allowed while this thread captures one
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        e = cudaHostRegister(g_gave_up, sizeof g_gave_up, cudaHostRegisterPortable | cudaHostRegisterMapped);
+        if (e == cudaErrorHostMemoryAlreadyRegistered) {       // another thread was faster
+            cudaGetLastError();
+            e = cudaSuccess;
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer(&base, g_gave_up, 0);
+    }
+    if (e != cudaSuccess || !base) {
+        cudaGetLastError();
+        return set_error(BI_ECUDA, "wait report: %s", cudaGetErrorString(e));
+    }
+    *word = static_cast<uint32_t*>(base) + line * 16;
+    return BI_OK;
+}
+
+bi_status waits_ok() {
+    const int line = gave_up_line();
+    if (line < 0 || *reinterpret_cast<volatile uint32_t*>(g_gave_up[line]) == 0) return BI_OK;
+    return set_error(BI_ETIMEDOUT, "a device wait of an earlier call ran out: results since then are incomplete "
+                                   "(bi_wait_status clears this)");
+}
+
 // CTAs an SM holds of a kernel that allocates tensor memory, from its
 // registers, shared memory and accumulator columns (the runtime's occupancy
 // query answers 1 for every such kernel).
@@ -165,6 +211,7 @@ static bi_status host_pipelined(const HostIO& io, uint64_t n, Launch launch) {
         if (rs == BI_OK && e != cudaSuccess) rs = cuda_ok(e, "pipeline");
         cudaStreamDestroy(st[k]);
     }
+    if (rs == BI_OK) rs = waits_ok();
     return rs;
 }
 
@@ -199,6 +246,7 @@ static bool run_in_place(const HostIO& io, uint64_t n, Launch launch, bi_status*
     *rs = launch(d[0], d[1], d[2], d[3], (uint8_t*)d[4], n, st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (*rs == BI_OK && e != cudaSuccess) *rs = cuda_ok(e, "in-place host launch");
+    if (*rs == BI_OK) *rs = waits_ok();
     cudaStreamDestroy(st);
     return true;
 }
@@ -334,6 +382,13 @@ const char* bi_status_string(bi_status s) {
 }
 
 const char* bi_last_error(void) { return g_err; }
+
+bi_status bi_wait_status(int clear) {
+    const bi_status st = waits_ok();
+    const int line = gave_up_line();
+    if (clear && line >= 0) *reinterpret_cast<volatile uint32_t*>(g_gave_up[line]) = 0;
+    return st;
+}
 
 // ---- the Futhark library's 1-D entries: one instance through the host twins
 bi_status bi_test_add_u64(const uint64_t* u, const uint64_t* v, uint64_t* w, uint32_t m) {

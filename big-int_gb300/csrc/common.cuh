@@ -107,6 +107,12 @@ __device__ __forceinline__ uint32_t block_carry_in(uint32_t g, uint32_t p, bool 
     return (warp_carry_resolve(A, B, cin).carries >> lane) & 1u;
 }
 
+// A wait ran out: the host finds it in `word` (host memory, see gave_up_word).
+__device__ __forceinline__ void report_gave_up(uint32_t* word) {
+    *reinterpret_cast<volatile uint32_t*>(word) = 1;
+    __threadfence_system();
+}
+
 }  // namespace bi
 
 // ---------------------------------------------------------------------------
@@ -123,6 +129,11 @@ bi_status set_error(bi_status st, const char* fmt, ...);
 bi_status check_launch(const char* what);
 int num_sms();
 cudaError_t smem_opt_in(const void* func, size_t smem);
+// Bounded waits (multc.cuh, addsub.cu): the current device's word that a kernel
+// sets where a wait of its ran out, and BI_ETIMEDOUT from then on until
+// bi_wait_status clears it.
+bi_status gave_up_word(uint32_t** word);
+bi_status waits_ok();
 int tc_ctas_per_sm(const void* kern, uint32_t threads, size_t smem, uint32_t cols);
 // products of at most 160 (full) or 256 (truncated) limbs, one warp each (mulmma.cu)
 bi_status mul_mma(const void* a, const void* b, void* r, uint32_t m, uint64_t n, bool w32, bool full, cudaStream_t st);

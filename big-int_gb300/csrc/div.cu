@@ -485,6 +485,7 @@ static bi_status div_entry(const T* u, const T* v, T* q, T* r, uint8_t* status, 
     if (method == DIV_SHINV && g.MU > DIV_SHINV_MAX_MU64)
         return set_error(BI_EUNSUPPORTED, "div_shinv: dividend of %u limbs above %u 64-bit limbs", mu,
                          DIV_SHINV_MAX_MU64);
+    BI_RETURN_IF(waits_ok());
     if (method != DIV_SHINV && g.MV <= (uint32_t)DIV_THREAD_MAX_MV) {
         launch_div_thread(u, v, q, r, status, mu, mv, n, (cudaStream_t)s);
         return check_launch("div thread kernel");

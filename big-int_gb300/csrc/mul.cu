@@ -376,8 +376,6 @@ static bi_status mul_thread(const T* a, const T* b, T* r, uint32_t m, uint64_t n
 // instance on the tensor core alone, 44.6K measured), 2.65 ms on the CTA
 // kernel's integer pipe.
 // ---------------------------------------------------------------------------
-__device__ uint32_t tc_gave_up;    // waits on the tensor core that ran out (never seen)
-
 template <typename T>
 struct TcRow {                         // an instance of a uniform batch
     const T *pa, *pb;
@@ -402,9 +400,9 @@ struct TcRow {                         // an instance of a uniform batch
 template <typename T, int P>
 __global__ void __launch_bounds__(TcShape<P>::THREADS, 1)
 mul_tc_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ r, uint64_t n, TcGeom g, uint32_t m,
-              uint32_t out_words, uint32_t out_limbs) {
+              uint32_t out_words, uint32_t out_limbs, uint32_t* gave_up) {
     extern __shared__ __align__(128) uint8_t smem_tc[];
-    tc_products<P>(g, smem_tc, blockIdx.x, gridDim.x, n, &tc_gave_up, [&](uint64_t inst) {
+    tc_products<P>(g, smem_tc, blockIdx.x, gridDim.x, n, gave_up, [&](uint64_t inst) {
         return TcRow<T>{a + inst * m, b + inst * m, r + inst * out_words, m, g.L, out_words, out_limbs};
     });
 }
@@ -420,8 +418,11 @@ static bi_status mul_tc_launch(const T* a, const T* b, T* r, uint32_t m, uint64_
     auto kern = mul_tc_kernel<T, P>;
     cudaError_t e = smem_opt_in((const void*)kern, smem);
     if (e != cudaSuccess) return set_error(BI_ECUDA, "mul: %s", cudaGetErrorString(e));
+    uint32_t* gave_up;
+    BI_RETURN_IF(gave_up_word(&gave_up));
     const uint64_t cap = (uint64_t)num_sms() * tc_ctas_per_sm((const void*)kern, TcShape<P>::THREADS, smem, TcShape<P>::TMEM_COLS);
-    kern<<<(unsigned)(n < cap ? n : cap), TcShape<P>::THREADS, smem, st>>>(a, b, r, n, g, m, out_words, out_limbs);
+    kern<<<(unsigned)(n < cap ? n : cap), TcShape<P>::THREADS, smem, st>>>(a, b, r, n, g, m, out_words, out_limbs,
+                                                                                           gave_up);
     return check_launch("mul tensor kernel");
 }
 
@@ -590,6 +591,7 @@ static bi_status mul_entry(const T* a, const T* b, T* r, uint32_t m, uint64_t n,
     if (!a || !b || !r) return set_error(BI_EINVAL, "NULL buffer");
     if ((uintptr_t)a % sizeof(T) || (uintptr_t)b % sizeof(T) || (uintptr_t)r % sizeof(T))
         return set_error(BI_EINVAL, "buffers must be aligned to the limb size");
+    BI_RETURN_IF(waits_ok());
     return mul_launch<T, FULL>(a, b, r, m, n, (cudaStream_t)s);
 }
 
@@ -603,6 +605,7 @@ static bi_status mul_chain(const T* a, const T* b, T* r, uint32_t m, uint64_t n,
         return set_error(BI_EINVAL, "buffers must be aligned to the limb size");
     const uint32_t L = sizeof(T) == 8 ? m : (m + 1) / 2;
     if (L > MUL_MAX_L) return set_error(BI_EUNSUPPORTED, "mul chain: m=%u above the supported size", m);
+    BI_RETURN_IF(waits_ok());
     MulGeom g = mul_geom_for<T, false>(L, n);   // the uniform multiply's tiling (128-thread CTAs unless tuned)
     g.S = 1;                                     // the chain kernel does not slice rows
     g.lgS = 0;
@@ -721,6 +724,7 @@ static bi_status mul_autotune_entry(const T* a, const T* b, T* r, uint32_t m, ui
         return set_error(BI_EINVAL, "buffers must be aligned to the limb size");
     const uint32_t L = sizeof(T) == 8 ? m : (m + 1) / 2;
     if (L > MUL_MAX_L) return set_error(BI_EUNSUPPORTED, "mul: m=%u above the supported size", m);
+    BI_RETURN_IF(waits_ok());
     return full ? mul_autotune<T, true>(a, b, r, m, n, reps, chosen, (cudaStream_t)s)
                 : mul_autotune<T, false>(a, b, r, m, n, reps, chosen, (cudaStream_t)s);
 }

@@ -130,8 +130,8 @@ __device__ __forceinline__ void tc_warp_arrive(uint32_t bar) {
         asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared::cta.b64 t, [%0];\n\t}" ::"r"(bar) : "memory");
 }
 
-// Waits for the barrier's phase; false after a second (the caller then waits
-// for nothing more and gives the results up).
+// Waits for the barrier's phase; false after a second (the caller then gives the
+// results up, reports it and leaves with nothing of its own in flight).
 __device__ __forceinline__ bool tc_bar_wait(uint32_t bar, uint32_t parity) {
     uint64_t t0 = 0;
     for (uint32_t tries = 0;; tries++) {
@@ -278,11 +278,13 @@ __device__ __forceinline__ void tc_free(uint32_t tmem) {
 //   issuing   the matrix instructions, into NS accumulators in turn;
 //   draining  each finished accumulator into 32-bit sums, then the product's
 //             limbs, while the tensor core is on the next blocks or instance.
+// HELD > 0 (a test) makes the barriers of B's stages wait for an arrival that
+// never comes.
 // fetch(i) gives instance i: L (at most g.L) and out_limbs, a(x) and b(x) the
 // limbs of its operands (x < L), store(x, v) takes limb x < out_limbs of its
 // product mod B^out_limbs.  Each role fetches an instance while it works on
-// the one before.  Every wait gives up after a second; the CTA then leaves and the call is
-// counted in `gave_up`.
+// the one before.  Every wait gives up after a second; a warp whose wait ran out
+// fills, issues and stores nothing more, the CTA leaves and reports to `gave_up`.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t tc_carry_in(uint32_t g, uint32_t p, uint32_t nwarps, uint32_t* scratch) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -298,7 +300,7 @@ __device__ __forceinline__ uint32_t tc_carry_in(uint32_t g, uint32_t p, uint32_t
     return (warp_carry_resolve(A, B, cin).carries >> lane) & 1u;
 }
 
-template <int P, typename Fetch>
+template <int P, uint32_t HELD = 0, typename Fetch>
 __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint64_t first, uint64_t step, uint64_t n,
                                             uint32_t* gave_up, Fetch fetch) {
     using S = TcShape<P>;
@@ -320,7 +322,7 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
     tc_fence_smem();
     const uint32_t tmem = tc_alloc<S::TMEM_COLS>(done + 8, [&] {
         for (uint32_t k = 0; k < NS; k++) {
-            tc_bar_init(made + 8 * k, 1);
+            tc_bar_init(made + 8 * k, 1 + HELD);
             tc_bar_init(run + 8 * k, 1);
             tc_bar_init(read + 8 * k, ND / 32);
         }
@@ -342,6 +344,7 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
             const auto next = fetch(i + step < n ? i + step : i);
             const uint32_t buf = p % g.NA;
             ok = tc_warp_wait(a_empty + 8 * buf, ((p / g.NA) & 1) ^ 1);
+            if (!ok) break;
             uint8_t* as = smem + buf * lay.abytes - g.rho0 * 16;
             uint64_t* bs = reinterpret_cast<uint64_t*>(smem + lay.braw + buf * lay.bbytes) + S::PAD;
 #pragma unroll 4
@@ -380,6 +383,7 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
                     for (int k0 = klo; k0 <= khi && ok; k0 += S::RB, c++) {
                         if (c % 4 != own) continue;
                         ok = tc_warp_wait(run + 8 * (c % NS), ((c / NS) & 1) ^ 1);
+                        if (!ok) break;
                         // core matrix x, row j0: bytes j0 - 7 .. j0 of limb w = Q - 1 - Q k0 - x,
                         // last first; they lie in three words, `sel` bytes into the first
                         const uint32_t* src = bs + 2 * (Q - 2 - Q * k0 - (int)(t >> 3));
@@ -396,7 +400,7 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
                         tc_warp_arrive(made + 8 * (c % NS));
                     }
                 }
-                tc_warp_arrive(a_empty + 8 * buf);     // b's limbs are read
+                if (ok) tc_warp_arrive(a_empty + 8 * buf);     // b's limbs are read
                 cur = next;
             }
         } else {
@@ -525,7 +529,7 @@ __device__ __forceinline__ void tc_products(const TcGeom& g, uint8_t* smem, uint
             cur = next;
         }
     }
-    if (!ok) atomicAdd(gave_up, 1u);
+    if (!ok) report_gave_up(gave_up);
     tc_free<S::TMEM_COLS>(tmem);
 }
 

@@ -197,7 +197,7 @@ static bi_status check_args(const void* a, const void* b, const void* r, uint32_
     if ((uintptr_t)a % sizeof(T) || (uintptr_t)b % sizeof(T) || (uintptr_t)r % sizeof(T))
         return set_error(BI_EINVAL, "buffers must be aligned to the limb size");
     if (n * (uint64_t)m > (1ull << 46)) return set_error(BI_EINVAL, "n*m too large");
-    return BI_OK;
+    return waits_ok();
 }
 
 static unsigned warp_grid(uint64_t n) {

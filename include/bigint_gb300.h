@@ -25,7 +25,12 @@
  *     drops the remainder, cuda/main.cu:135,307) every instance is computed;
  *   - device buffers need the natural alignment of their limb type; 16-byte
  *     aligned buffers take the vectorised path;
- *   - calls are thread-safe; concurrent calls on different streams overlap.
+ *   - calls are thread-safe; concurrent calls on different streams overlap;
+ *   - every device-side wait has a limit (a second).  Where one runs out the
+ *     kernel ends without the results that it waited for, and bi_wait_status
+ *     and every later call that would launch work on that device return
+ *     BI_ETIMEDOUT, launching nothing, until bi_wait_status clears it (the
+ *     bi_host_* calls and bi_batch_run_noalloc report their own waits).
  */
 #ifndef BIGINT_GB300_H
 #define BIGINT_GB300_H
@@ -54,6 +59,11 @@ const char* bi_status_string(bi_status status);
 
 /* Detail text of the last failing call on the calling thread ("" if none). */
 const char* bi_last_error(void);
+
+/* BI_ETIMEDOUT if a device wait of a kernel that has ended ran out on the */
+/* current device (synchronise the stream first to know of its calls),    */
+/* else BI_OK; clear != 0 resets it.                                      */
+bi_status bi_wait_status(int clear);
 
 /* Library version as 10000*major + 100*minor + patch. */
 int bi_version(void);
@@ -500,6 +510,15 @@ bi_status bi_fill_splitmix64(uint64_t* dst, uint64_t count, uint64_t seed,
 /* Synchronous on `stream`.                                                */
 /* ---------------------------------------------------------------------- */
 bi_status bi_probe_intpipe(double* rates, bi_stream stream);
+
+/* ---------------------------------------------------------------------- */
+/* What a device wait that runs out does (for tests): a kernel on a barrier */
+/* that never completes.  It ends by its own limit, leaves r as it was and  */
+/* makes bi_wait_status BI_ETIMEDOUT.  kind 0: full products of m <= 128    */
+/* limbs, r is [n][2m]; 2 <= n <= 64.                                       */
+/* ---------------------------------------------------------------------- */
+bi_status bi_probe_held_wait(int kind, const uint64_t* a, const uint64_t* b, uint64_t* r, uint8_t* status,
+                             uint32_t m, uint64_t n, bi_stream stream);
 
 #ifdef __cplusplus
 }
