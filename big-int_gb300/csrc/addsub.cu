@@ -529,7 +529,8 @@ addsub_chunk_kernel(const T* a, const T* b, T* r, uint8_t* sign_out, uint32_t cp
 // which meets every bank once, and the tile goes back as vectors, its ends limb
 // by limb.  An instance's last chunk is padded with zeros, which pass a borrow
 // on.  r may be a or b: a tile's limbs are written by its own CTA alone, after
-// they have come.
+// they have come.  HELD > 0 (a test): the copies' barriers wait for bytes that
+// never come.
 //
 // Bound by HBM: 5.8-6.4 TB/s against the row kernel's 3.0 (u32) and 4.5 (u64)
 // for differences, whose two borrow chains a row it resolves limb by limb with
@@ -538,7 +539,7 @@ addsub_chunk_kernel(const T* a, const T* b, T* r, uint8_t* sign_out, uint32_t cp
 // tiles staged through registers instead of by bulk copies ran at 110-150 us
 // where this takes 66-75 (400 MB), with nothing in flight between barriers.
 // ---------------------------------------------------------------------------
-template <typename T, int W, int K, int OP>
+template <typename T, int W, int K, int OP, uint32_t HELD = 0>
 __global__ void __launch_bounds__(W * 32)
 addsub_ragged_kernel(const T* a, const T* b, T* r, uint8_t* sign_out, uint32_t m, uint32_t cpi, uint64_t n, uint32_t ipt,
                      uint64_t ntiles, uint32_t* gave_up) {
@@ -583,7 +584,8 @@ addsub_ragged_kernel(const T* a, const T* b, T* r, uint8_t* sign_out, uint32_t m
     auto fetch = [&](uint64_t tile, int st) {                   // one thread
         const Tile t = tile_at(tile);
         const uint32_t bytes = (uint32_t)(t.bulk * sizeof(T)), bar = bars + 8 * st;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * bytes) : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * bytes + 16 * HELD)
+                     : "memory");
         if (bytes == 0) return;
 #pragma unroll
         for (int k = 0; k < 2; k++)
@@ -612,6 +614,11 @@ addsub_ragged_kernel(const T* a, const T* b, T* r, uint8_t* sign_out, uint32_t m
         const bool valid = q < t.ninst;
         const bool ok = tc_bar_wait(bars + 8 * st, (it >> 1) & 1);
         if (__syncthreads_or(!ok)) {
+            // The CTA leaves only when no copy into its shared memory, which the
+            // SM's next CTA gets, is under way: this tile's and the next one's
+            // (the one after that is not asked for yet) are waited for once more.
+            tc_bar_wait(bars + 8 * st, (it >> 1) & 1);
+            if (tile + gridDim.x < ntiles) tc_bar_wait(bars + 8 * (st ^ 1), ((it + 1) >> 1) & 1);
             if (threadIdx.x == 0) report_gave_up(gave_up);
             return;
         }
@@ -866,6 +873,18 @@ static bi_status launch_ragged(const T* a, const T* b, T* r, uint8_t* sign, uint
     const uint64_t cap = (uint64_t)num_sms() * occ;
     kern<<<(unsigned)(ntiles < cap ? ntiles : cap), W * 32, smem, st>>>(a, b, r, sign, m, cpi, n, ipt, ntiles, gave_up);
     return check_launch(OP == OP_ADD ? "add kernel" : "sub kernel");
+}
+
+bi_status ragged_held(const uint64_t* a, const uint64_t* b, uint64_t* r, uint8_t* sign, uint32_t m, uint64_t n,
+                      uint32_t* gave_up, cudaStream_t st) {
+    constexpr int W = 8, K = 7;
+    const uint32_t cpi = (m + K - 1) / K, ipt = W * 32 / cpi;
+    const size_t smem = 4 * (W * 32 * K + 4) * sizeof(uint64_t);
+    auto kern = addsub_ragged_kernel<uint64_t, W, K, OP_SUB, 1>;
+    cudaError_t e = smem_opt_in((const void*)kern, smem);
+    if (e != cudaSuccess) return set_error(BI_ECUDA, "held wait: %s", cudaGetErrorString(e));
+    kern<<<1, W * 32, smem, st>>>(a, b, r, sign, m, cpi, n, ipt, (n + ipt - 1) / ipt, gave_up);
+    return check_launch("held sub kernel");
 }
 
 // ---------------------------------------------------------------------------

@@ -134,6 +134,9 @@ cudaError_t smem_opt_in(const void* func, size_t smem);
 // bi_wait_status clears it.
 bi_status gave_up_word(uint32_t** word);
 bi_status waits_ok();
+// the ragged difference kernel on a barrier that never completes (waitprobe.cu)
+bi_status ragged_held(const uint64_t* a, const uint64_t* b, uint64_t* r, uint8_t* sign, uint32_t m, uint64_t n,
+                      uint32_t* gave_up, cudaStream_t st);
 int tc_ctas_per_sm(const void* kern, uint32_t threads, size_t smem, uint32_t cols);
 // products of at most 160 (full) or 256 (truncated) limbs, one warp each (mulmma.cu)
 bi_status mul_mma(const void* a, const void* b, void* r, uint32_t m, uint64_t n, bool w32, bool full, cudaStream_t st);

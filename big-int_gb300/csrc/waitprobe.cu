@@ -45,7 +45,10 @@ extern "C" bi_status bi_probe_held_wait(int kind, const uint64_t* a, const uint6
     BI_RETURN_IF(waits_ok());
     uint32_t* gave_up;
     BI_RETURN_IF(gave_up_word(&gave_up));
-    (void)status;
     if (kind == 0) return held_products(a, b, r, m, n, gave_up, (cudaStream_t)s);
+    if (kind == 1) {
+        if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)r) % 16) return set_error(BI_EINVAL, "held wait: buffers off a 16-byte boundary");
+        return ragged_held(a, b, r, status, m, n, gave_up, (cudaStream_t)s);
+    }
     return set_error(BI_EINVAL, "held wait: no kind %d", kind);
 }

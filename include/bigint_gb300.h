@@ -515,7 +515,8 @@ bi_status bi_probe_intpipe(double* rates, bi_stream stream);
 /* What a device wait that runs out does (for tests): a kernel on a barrier */
 /* that never completes.  It ends by its own limit, leaves r as it was and  */
 /* makes bi_wait_status BI_ETIMEDOUT.  kind 0: full products of m <= 128    */
-/* limbs, r is [n][2m]; 2 <= n <= 64.                                       */
+/* limbs, r is [n][2m]; 1: differences by bulk copies, r is [n][m], status  */
+/* takes their signs; 2 <= n <= 64.                                         */
 /* ---------------------------------------------------------------------- */
 bi_status bi_probe_held_wait(int kind, const uint64_t* a, const uint64_t* b, uint64_t* r, uint8_t* status,
                              uint32_t m, uint64_t n, bi_stream stream);

@@ -67,6 +67,21 @@ def test_products(waits, oracle, m, n):
     _check_reported(B, oracle)
 
 
+@pytest.mark.parametrize("m,n", [(7, 2), (125, 64)])
+def test_differences(waits, oracle, m, n):
+    """One tile, and five on one CTA with the next one's copies under way."""
+    import torch
+
+    B = waits
+    a, b = B.to_device(uniform_limbs(3, n, m)), B.to_device(uniform_limbs(4, n, m))
+    r = torch.full((n, m), 77, dtype=torch.int64, device="cuda")
+    sign = torch.full((n,), 77, dtype=torch.uint8, device="cuda")
+    _held(B, 1, a, b, r, sign, m, n)
+    assert bool((r == 77).all()) and bool((sign == 77).all())
+    _check_reported(B, oracle)
+    assert (B.to_host(B.sub(a, b)[0], np.uint64) == oracle.sub(B.to_host(a, np.uint64), B.to_host(b, np.uint64))[0]).all()
+
+
 def test_plan_is_refused(waits):
     import torch
 
