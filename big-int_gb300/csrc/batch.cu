@@ -458,12 +458,11 @@ batch_divblk_kernel(const bi_desc* __restrict__ descs, const uint32_t* __restric
 template <int P, int G>
 __global__ void __launch_bounds__(DtShape<P, G>::NT)
 batch_divtc_kernel(const bi_desc* __restrict__ descs, const uint32_t* __restrict__ list, uint32_t count,
-                   uint32_t* counter, const uint64_t* in, uint64_t* out, uint8_t* flags, uint32_t mu) {
+                   uint32_t* counter, const uint64_t* in, uint64_t* out, uint8_t* flags, uint32_t mu, uint32_t* gave_up) {
     extern __shared__ __align__(128) uint8_t smem_dt[];
     __shared__ uint32_t s_idx;
     const DtSmem<P, G> lay(dt_geom(mu, 1, 8));
-    const uint32_t bar = tc_smem_addr(smem_dt) + lay.bar;
-    const uint32_t tmem = tc_alloc<DtShape<P, G>::TMEM_COLS>(bar + 8, [&] { tc_bar_init(bar, 1); });
+    const uint32_t tmem = dt_begin<P, G>(lay, smem_dt);
     uint32_t phase = 0;
     for (;;) {
         if (threadIdx.x == 0) s_idx = atomicAdd(counter, 1u);
@@ -480,7 +479,7 @@ batch_divtc_kernel(const bi_desc* __restrict__ descs, const uint32_t* __restrict
         const uint8_t st = dt_divide<P, G>(dt_geom(m64(d), mb64(d), 8), lay, smem_dt, tmem, phase, lu, lv, sq, sr);
         if (flags && threadIdx.x == 0) flags[d.flag] = st;
     }
-    tc_free<DtShape<P, G>::TMEM_COLS>(tmem);
+    dt_end<P, G>(lay, smem_dt, tmem, gave_up);
 }
 
 struct bi_plan {
@@ -833,11 +832,11 @@ static bi_status launch_plan_kernels(bi_plan* p, const uint64_t* in, uint64_t* o
             case 8: batch_divwarp_kernel<16><<<grid, DIV_WARP_CTA, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             case 9: batch_divwarp3_kernel<24><<<grid, DIV_WARP_CTA, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             case 10: batch_divwarp_kernel<32><<<grid, DIV_WARP_CTA, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
-            case DIV_TC0: batch_divtc_kernel<16, 1><<<grid, DtShape<16, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[0]); break;
-            case DIV_TC0 + 1: batch_divtc_kernel<32, 1><<<grid, DtShape<32, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[1]); break;
-            case DIV_TC0 + 2: batch_divtc_kernel<64, 1><<<grid, DtShape<64, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[2]); break;
-            case DIV_TC0 + 3: batch_divtc_kernel<80, 2><<<grid, DtShape<80, 2>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[3]); break;
-            case DIV_TC0 + 4: batch_divtc_kernel<128, 1><<<grid, DtShape<128, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[4]); break;
+            case DIV_TC0: batch_divtc_kernel<16, 1><<<grid, DtShape<16, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[0], gave_up); break;
+            case DIV_TC0 + 1: batch_divtc_kernel<32, 1><<<grid, DtShape<32, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[1], gave_up); break;
+            case DIV_TC0 + 2: batch_divtc_kernel<64, 1><<<grid, DtShape<64, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[2], gave_up); break;
+            case DIV_TC0 + 3: batch_divtc_kernel<80, 2><<<grid, DtShape<80, 2>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[3], gave_up); break;
+            case DIV_TC0 + 4: batch_divtc_kernel<128, 1><<<grid, DtShape<128, 1>::NT, L.smem[2 + c], st>>>(p->d_descs, list, n, ctr, in, out, flags, p->divc_mu[4], gave_up); break;
             case DIV_BLK2_CLASS: batch_divblk_kernel<2><<<grid, 64, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             case DIV_BLK4_CLASS: batch_divblk_kernel<4><<<grid, 128, 0, st>>>(p->d_descs, list, n, ctr, in, out, flags); break;
             default:

@@ -134,7 +134,9 @@ cudaError_t smem_opt_in(const void* func, size_t smem);
 // bi_wait_status clears it.
 bi_status gave_up_word(uint32_t** word);
 bi_status waits_ok();
-// the ragged difference kernel on a barrier that never completes (waitprobe.cu)
+// the ragged difference and the block division kernel on a barrier that never completes (waitprobe.cu)
+bi_status div_held(const uint64_t* u, const uint64_t* v, uint64_t* q, uint64_t* r, uint8_t* status, uint32_t mu,
+                   uint32_t mv, uint64_t n, uint32_t* gave_up, cudaStream_t st);
 bi_status ragged_held(const uint64_t* a, const uint64_t* b, uint64_t* r, uint8_t* sign, uint32_t m, uint64_t n,
                       uint32_t* gave_up, cudaStream_t st);
 int tc_ctas_per_sm(const void* kern, uint32_t threads, size_t smem, uint32_t cols);

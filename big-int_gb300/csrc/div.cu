@@ -393,14 +393,13 @@ static void launch_div_blk(const T* u, const T* v, T* q, T* r, uint8_t* status, 
 // (P = 16 held to 12 CTAs an SM, 40 registers: 192-limb divisors 376 -> 347 us at
 // 10922, 128-limb ones 418 -> 403; wider shapes ran slower so.  0 leaves the bound to
 // the compiler, 64 to 96 registers; a 1 lets it take 250: 1024 limbs 565 -> 930 us)
-template <typename T, int P, int G>
+template <typename T, int P, int G, uint32_t HELD = 0>
 __global__ void __launch_bounds__(DtShape<P, G>::NT, P == 16 ? 12 : 0)
 div_tc_kernel(const T* __restrict__ u, const T* __restrict__ v, T* __restrict__ q, T* __restrict__ r,
-              uint8_t* __restrict__ status, uint64_t n, DtGeom g) {
+              uint8_t* __restrict__ status, uint64_t n, DtGeom g, uint32_t* gave_up) {
     extern __shared__ __align__(128) uint8_t smem_dt[];
     const DtSmem<P, G> lay(g);
-    const uint32_t bar = tc_smem_addr(smem_dt) + lay.bar;
-    const uint32_t tmem = tc_alloc<DtShape<P, G>::TMEM_COLS>(bar + 8, [&] { tc_bar_init(bar, 1); });
+    const uint32_t tmem = dt_begin<P, G, HELD>(lay, smem_dt);
     uint32_t phase = 0;
     for (uint64_t inst = blockIdx.x; inst < n; inst += gridDim.x) {
         const T* ui = u + inst * g.mu;
@@ -413,7 +412,7 @@ div_tc_kernel(const T* __restrict__ u, const T* __restrict__ v, T* __restrict__ 
             [&](uint32_t i, uint64_t x) { put_limb64(ri, g.mv, i, x); });
         if (status && threadIdx.x == 0) status[inst] = st;
     }
-    tc_free<DtShape<P, G>::TMEM_COLS>(tmem);
+    dt_end<P, G>(lay, smem_dt, tmem, gave_up);
 }
 
 template <typename T, int P, int G>
@@ -423,9 +422,22 @@ static bi_status launch_div_tc(const T* u, const T* v, T* q, T* r, uint8_t* stat
     auto kern = div_tc_kernel<T, P, G>;
     cudaError_t e = smem_opt_in((const void*)kern, smem);
     if (e != cudaSuccess) return set_error(BI_ECUDA, "div: %s", cudaGetErrorString(e));
+    uint32_t* gave_up;
+    BI_RETURN_IF(gave_up_word(&gave_up));
     const uint64_t cap = (uint64_t)num_sms() * tc_ctas_per_sm((const void*)kern, DtShape<P, G>::NT, smem, DtShape<P, G>::TMEM_COLS);
-    kern<<<(unsigned)(n < cap ? n : cap), DtShape<P, G>::NT, smem, s>>>(u, v, q, r, status, n, g);
+    kern<<<(unsigned)(n < cap ? n : cap), DtShape<P, G>::NT, smem, s>>>(u, v, q, r, status, n, g, gave_up);
     return check_launch("div tensor kernel");
+}
+
+bi_status div_held(const uint64_t* u, const uint64_t* v, uint64_t* q, uint64_t* r, uint8_t* status, uint32_t mu,
+                   uint32_t mv, uint64_t n, uint32_t* gave_up, cudaStream_t s) {
+    const DtGeom g = dt_geom(mu, mv, 8);
+    const size_t smem = DtSmem<16, 1>(g).total;
+    auto kern = div_tc_kernel<uint64_t, 16, 1, 1>;
+    cudaError_t e = smem_opt_in((const void*)kern, smem);
+    if (e != cudaSuccess) return set_error(BI_ECUDA, "held wait: %s", cudaGetErrorString(e));
+    kern<<<2, DtShape<16, 1>::NT, smem, s>>>(u, v, q, r, status, n, g, gave_up);
+    return check_launch("held div kernel");
 }
 
 // the narrowest accumulator whose rows hold the divisor

@@ -85,7 +85,7 @@ struct DtSmem {
         cs = qh + (S::LW + 2) * 8;
         scratch = cs + (S::NT + 1) * 8;
         bar = scratch + 3 * 32 * 4;
-        total = bar + 16;
+        total = bar + 16;      // the barrier, tensor memory's address, whether a wait ran out
     }
 };
 
@@ -364,7 +364,8 @@ __device__ __forceinline__ void dt_recip(const uint64_t* v, uint64_t* y, uint64_
 // store_q(i, x) for i < g.MU and store_r(i, x) for i < g.MV receive the
 // results.  `phase` is the barrier's.  Every thread of the CTA calls it and
 // gets the status: 0, 1 for a zero divisor, 2 when the corrections or a wait
-// ran out.
+// ran out.  After a wait that ran out the CTA's barrier may be behind `phase`: its
+// later divisions wait no more and are 2 as well (dt_end has the rest).
 template <int P, int G, typename LoadU, typename LoadV, typename StoreQ, typename StoreR>
 __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P, G>& lay, uint8_t* smem, uint32_t tmem,
                                              uint32_t& phase, LoadU load_u, LoadV load_v, StoreQ store_q,
@@ -458,7 +459,8 @@ __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P, G>
     }
     __syncthreads();
 
-    bool ok = true;
+    volatile uint32_t* lost = reinterpret_cast<volatile uint32_t*>(smem + lay.bar + 12);
+    bool ok = *lost == 0;
     int fixes = 0;
     for (int blk = nb - 1; blk >= 0; blk--) {
         const int w0 = blk * KB;          // the window: limbs w0 .. w0 + Kp + 30
@@ -687,7 +689,50 @@ __device__ __forceinline__ uint8_t dt_divide(const DtGeom& g, const DtSmem<P, G>
         }
         store_r((uint32_t)i, x);
     }
+    if (!ok) *lost = 1;
     return __syncthreads_or(!ok || fixes) ? 2 : 0;
+}
+
+// The barrier and tensor memory of a CTA that divides, before and after all its
+// divisions.  HELD > 0 (a test): the barrier waits for an arrival that never comes.
+template <int P, int G, uint32_t HELD = 0>
+__device__ __forceinline__ uint32_t dt_begin(const DtSmem<P, G>& lay, uint8_t* smem) {
+    const uint32_t bar = tc_smem_addr(smem) + lay.bar;
+    return tc_alloc<DtShape<P, G>::TMEM_COLS>(bar + 8, [&] {
+        tc_bar_init(bar, 1 + HELD);
+        *reinterpret_cast<volatile uint32_t*>(smem + lay.bar + 12) = 0;
+    });
+}
+
+// A wait ran out: waits, with the same limit, until all that the CTA issued has
+// ended, and tells the host.  `at` is a free word of shared memory.
+__device__ __forceinline__ void dt_settle(uint32_t at, uint32_t* gave_up) {
+    if (threadIdx.x == 0) {
+        report_gave_up(gave_up);
+        tc_bar_init(at, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (__shfl_sync(0xffffffffu, threadIdx.x >> 5, 0) == 0) {
+        if (tc_elect()) tc_commit(at);         // by the thread that issues: all it issued
+        __syncwarp();
+    }
+    tc_bar_wait(at, 0);
+}
+
+// (never run, but it moves the registers of the kernel's loop: 63-limb blocks keep
+// theirs with the call, 2048 by 1024 limbs 565 / 573 us, the others without it, 512
+// by 256 410 / 423)
+static __device__ __noinline__ void dt_settle_call(uint32_t at, uint32_t* gave_up) { dt_settle(at, gave_up); }
+
+template <int P, int G>
+__device__ __forceinline__ void dt_end(const DtSmem<P, G>& lay, uint8_t* smem, uint32_t tmem, uint32_t* gave_up) {
+    __syncthreads();
+    if (*reinterpret_cast<volatile uint32_t*>(smem + lay.bar + 12) != 0) {
+        if constexpr (G == 1) dt_settle(tc_smem_addr(smem) + lay.cs, gave_up);
+        else dt_settle_call(tc_smem_addr(smem) + lay.cs, gave_up);
+    }
+    tc_free<DtShape<P, G>::TMEM_COLS>(tmem);
 }
 
 }  // namespace bi

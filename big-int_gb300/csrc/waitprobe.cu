@@ -50,5 +50,6 @@ extern "C" bi_status bi_probe_held_wait(int kind, const uint64_t* a, const uint6
         if (((uintptr_t)a | (uintptr_t)b | (uintptr_t)r) % 16) return set_error(BI_EINVAL, "held wait: buffers off a 16-byte boundary");
         return ragged_held(a, b, r, status, m, n, gave_up, (cudaStream_t)s);
     }
+    if (kind == 2) return div_held(a, b, r, r + 2 * m * n, status, 2 * m, m, n, gave_up, (cudaStream_t)s);
     return set_error(BI_EINVAL, "held wait: no kind %d", kind);
 }

@@ -155,8 +155,9 @@ bi_status bi_mul_set_tuning_u32(uint32_t m, int full, int ipc, int slices);
 /* Futhark div / test_div (futhark/div.fut:150-167,                        */
 /* futhark/test/gmp-validation-lib.fut:26-27), which require equal sizes;  */
 /* here the divisor may be shorter.  status (may be NULL) is [n]:          */
-/* 0 = ok, 1 = divisor zero (q_i and r_i are set to 0), 2 = internal      */
-/* correction bound exceeded (never observed).  The reference divides by   */
+/* 0 = ok, 1 = divisor zero (q_i and r_i are set to 0), 2 = no result: an  */
+/* internal correction bound exceeded or a device wait that ran out        */
+/* (neither ever observed; for the second see bi_wait_status).  The reference divides by   */
 /* zero (div.c:165-181); this entry reports it per instance instead.       */
 /* q and r must not overlap u, v or each other.                            */
 /* mu <= bi_max_limbs_div_* () (8192 64-bit limbs), mv <= 4096 64-bit    */
@@ -513,10 +514,11 @@ bi_status bi_probe_intpipe(double* rates, bi_stream stream);
 
 /* ---------------------------------------------------------------------- */
 /* What a device wait that runs out does (for tests): a kernel on a barrier */
-/* that never completes.  It ends by its own limit, leaves r as it was and  */
+/* that never completes.  It ends by its own limit, leaves no result and    */
 /* makes bi_wait_status BI_ETIMEDOUT.  kind 0: full products of m <= 128    */
 /* limbs, r is [n][2m]; 1: differences by bulk copies, r is [n][m], status  */
-/* takes their signs; 2 <= n <= 64.                                         */
+/* takes their signs; 2: block division, a is [n][2m], r has the quotients  */
+/* [n][2m] and then the remainders [n][m]; 2 <= n <= 64.                    */
 /* ---------------------------------------------------------------------- */
 bi_status bi_probe_held_wait(int kind, const uint64_t* a, const uint64_t* b, uint64_t* r, uint8_t* status,
                              uint32_t m, uint64_t n, bi_stream stream);

@@ -82,6 +82,23 @@ def test_differences(waits, oracle, m, n):
     assert (B.to_host(B.sub(a, b)[0], np.uint64) == oracle.sub(B.to_host(a, np.uint64), B.to_host(b, np.uint64))[0]).all()
 
 
+@pytest.mark.parametrize("m,n", [(40, 2), (128, 24)])
+def test_divisions(waits, oracle, m, n):
+    """One division and twelve a CTA: status 2 for all, also those after the one that waited."""
+    import torch
+
+    B = waits
+    a, b = B.to_device(uniform_limbs(3, n, 2 * m)), B.to_device(uniform_limbs(4, n, m))
+    r = torch.full((3 * n * m,), 77, dtype=torch.int64, device="cuda")
+    status = torch.full((n,), 77, dtype=torch.uint8, device="cuda")
+    _held(B, 2, a, b, r, status, m, n)
+    assert bool((status == 2).all())
+    _check_reported(B, oracle)
+    q, rem, st = B.div(a, b)
+    wq, wr, ws = oracle.div(B.to_host(a, np.uint64), B.to_host(b, np.uint64))
+    assert (B.to_host(q, np.uint64) == wq).all() and (B.to_host(rem, np.uint64) == wr).all() and not st.any()
+
+
 def test_plan_is_refused(waits):
     import torch
 
