@@ -413,7 +413,8 @@ def measure_extra(B, L, stream, args):
                              "truncated_gu32ops_fft_normalised": round(gu32ops(n, 2 * m, ms_t), 1),
                              "autotuned_full_instances_per_s": round(n / ms_tuned * 1e3),
                              "autotuned_frac_of_intpipe_peak": round(wp / ms_tuned * 1e3 / peak_wps, 4),
-                             "autotuned_tiling": {"instances_per_cta": chosen[0], "row_slices": chosen[1]}}
+                             "autotuned_tiling": "tensor cores" if chosen[0] == B.MUL_DEFAULT else
+                             {"instances_per_cta": chosen[0], "row_slices": chosen[1]}}
         del a, b, r, rt
     out["mul_u64_full"] = mul
     a, b = mul2048_u32()
@@ -448,6 +449,7 @@ def measure_extra(B, L, stream, args):
         check(L, L.bi_mul_set_tuning_u64(m, 1, 0, 0))       # back to the library's own choice
         pick = ("warp kernel, 32-bit words" if (chosen[0], chosen[1]) == (0, 0) else
                 "thread kernel, 64-bit limbs" if (chosen[0], chosen[1]) == (0, 1) else
+                "tensor cores" if chosen[0] == B.MUL_DEFAULT else
                 f"CTA kernel, 64-bit limbs, {chosen[0]} instances x {chosen[1]} slices")
         small[f"m{m}_n{n}"] = {"instances_per_s": round(n / ms * 1e3), "word_products_per_s": wp / ms * 1e3,
                                "frac_of_intpipe_peak": round(wp / ms * 1e3 / peak_wps, 4),

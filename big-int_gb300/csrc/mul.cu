@@ -632,8 +632,9 @@ static bi_status mul_chain(const T* a, const T* b, T* r, uint32_t m, uint64_t n,
 // as {0, 1}, beside the CTA
 // kernel's tilings (64-bit limbs: row_mac8) -- the arithmetic's word width
 // and the threads an instance are part of what is tuned.  Where the call
-// would go to the tensor cores they are a candidate too, reported as {1, 1}, and
-// nothing is recorded when they are the fastest.
+// would go to the tensor cores they are a candidate too, reported as
+// {BI_MUL_DEFAULT, 1} (no tiling: setting that is setting nothing), and nothing is
+// recorded when they are the fastest.
 template <typename T, bool FULL>
 static bi_status mul_autotune(const T* a, const T* b, T* r, uint32_t m, uint64_t n, int reps, int* chosen,
                               cudaStream_t st) {
@@ -668,7 +669,7 @@ static bi_status mul_autotune(const T* a, const T* b, T* r, uint32_t m, uint64_t
     bi_status st_out = BI_OK;
     const int kind = mul_matrix_kernel(L, FULL, n);
     const size_t ntiled = cands.size();
-    if (kind != MUL_OTHER) cands.push_back({1, 1});
+    if (kind != MUL_OTHER) cands.push_back({BI_MUL_DEFAULT, 1});
     bool pick_matrix = false;
     for (size_t ci = 0; ci < cands.size(); ci++) {
         const auto& c = cands[ci];
@@ -736,7 +737,7 @@ static bi_status mul_set_tuning(int limb_bytes, uint32_t m, int full, int ipc, i
     int dev = 0;
     cudaGetDevice(&dev);
     const auto key = std::make_tuple(dev, limb_bytes, full ? 1 : 0, L);
-    if (ipc == 0) {                                   // back to the library's own choice
+    if (ipc == 0 || (ipc == BI_MUL_DEFAULT && slices == 1)) {   // back to the library's own choice
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tune.erase(key);
         return BI_OK;

@@ -129,15 +129,18 @@ bi_status bi_mulfull_u32(const uint32_t* a, const uint32_t* b, uint32_t* r,
 /* for this device, limb width, product kind (full != 0: bi_mulfull_*)    */
 /* and m, which later calls then use, and leaves r as that call writes    */
 /* it; synchronous on `stream`.  chosen (may be NULL) gets {instances per */
-/* CTA, slices} ({1, 1} for the tensor cores too, which stay the default), */
-/* or {0, 0} when the warp kernel was fastest, {0, 1} for                  */
-/* the thread kernel.  The reference fixes its tiling per size at compile */
+/* CTA, slices}, {BI_MUL_DEFAULT, 1} when the library's own choice, the    */
+/* tensor cores, was fastest (nothing is recorded then, and a tuning for m */
+/* is cleared), {0, 0} when the warp kernel was, {0, 1} for the thread     */
+/* kernel.  The reference fixes its tiling per size at compile */
 /* time (ipb and the Q limbs per thread, cuda/main.cu:15-28).             */
 /* bi_mul_set_tuning_* sets a tiling by hand (BI_EINVAL if it does not    */
 /* fit a CTA); ipc = -1 picks a per-instance kernel (slices = 0: the warp */
 /* kernel, full products of at most 32 limbs; 1: the thread kernel, full  */
-/* products of at most 24 limbs, truncated ones of at most 32); ipc = 0   */
-/* returns (m, full) to the library's own choice.                         */
+/* products of at most 24 limbs, truncated ones of at most 32); ipc = 0,  */
+/* or BI_MUL_DEFAULT with one slice, returns (m, full) to the library's   */
+/* own choice.                                                            */
+#define BI_MUL_DEFAULT 65536   /* more instances than any CTA holds */
 bi_status bi_mul_autotune_u64(const uint64_t* a, const uint64_t* b, uint64_t* r,
                               uint32_t m, uint64_t n, int full, int reps, int* chosen,
                               bi_stream stream);
