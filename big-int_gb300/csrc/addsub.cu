@@ -951,10 +951,20 @@ static bi_status addsub(const T* a, const T* b, T* r, uint8_t* sign, uint32_t m,
         // u64 251-276 / 330-362, sub u32 253-295 / 475-854, add u32 240-276 /
         // 274-495.  Below 5 (u32: 7) limbs most of a lane's chunk would be
         // padding: sub of 4 u64 limbs 98 / 99 us on 400 MB, of 6 u32 limbs 109 /
-        // 140 but add 87 / 81.
+        // 140 but add 87 / 81.  Rows of 8, 12 or 24 words have the lanes' chunks 8
+        // or 12 words apart, where 8 or 4 lanes meet in a bank: beyond a few
+        // thousand instances the row kernel takes the sums (ragged / row on 400
+        // MB: 8 words 121 / 69, 12 words 71.5 / 70, 24 words 77 / 70; 20000 of 8
+        // words 2.8 / 2.9) and differences of 8 words (135 / 125; 100000 of them
+        // 5.3 / 7.4).  Sums of 3841 to 4096 words too: there it still takes its
+        // 8-warp tile and this one 16 warps (3845 words 84 / 73, 4500 75 / 118).
         if constexpr (OP == OP_SUB || sizeof(T) == 4) {
             constexpr uint32_t KR = sizeof(T) == 8 ? 7 : 15, LO = sizeof(T) == 8 ? 5 : 7;
-            if (!host_link && m >= LO && m <= 16 * 32 * KR) {
+            const bool row = sizeof(T) == 4 &&
+                             (OP == OP_ADD ? ((m == 8 || m == 12 || m == 24) && n * m > (1u << 18)) ||
+                                                 (m > 8 * 32 * KR && m + 3 <= 8 * 4 * 32 * 4)
+                                           : m == 8 && n * m > (1u << 21));
+            if (!host_link && !row && m >= LO && m <= 16 * 32 * KR) {
                 if (m <= 8 * 32 * KR) return launch_ragged<T, 8, KR, OP>(a, b, r, sign, m, n, st);
                 return launch_ragged<T, 16, KR, OP>(a, b, r, sign, m, n, st);
             }
