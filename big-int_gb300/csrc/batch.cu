@@ -235,13 +235,20 @@ constexpr int PLAN_MULTC0 = PLAN_MULW0 + MULW_CLASSES;   // and of the first ten
 
 // Divisions whose quotient is long enough to earn back the block division's
 // setup (div.cu's rule for a batch that fills the GPU; up to 128 limbs the
-// lane groups pack better beside the batch's other kernels).
-static inline bool batch_div_on_tc(uint32_t m, uint32_t mv) {
-    return mv > 128 && mv <= (uint32_t)DtShape<128, 1>::MAX_K && (uint64_t)mv * (m - mv + 1) >= 9400;
+// lane groups pack better beside the batch's other kernels).  `shorts` is the
+// batch's number of divisions by 736 to 1024 limbs with short quotients
+// (div_short_quotient), counted if long division on warps, not the shifted
+// inverse, would take them (more than 6 an SM): 4864 of 1003 by 992 limbs alone
+// in a plan 243 us on the tensor cores, 154 on warps, 608 of them 41 and (shifted
+// inverse) 77.
+static inline bool batch_div_on_tc(uint32_t m, uint32_t mv, uint64_t shorts, int sms) {
+    const uint64_t ql = m - mv + 1;
+    return mv > 128 && mv <= (uint32_t)DtShape<128, 1>::MAX_K && mv * ql >= 9400 &&
+           !div_short_quotient(mv, ql, shorts, sms);
 }
 
-static inline int div_class(uint32_t m, uint32_t mv) {
-    if (batch_div_on_tc(m, mv)) {
+static inline int div_class(uint32_t m, uint32_t mv, uint64_t shorts, int sms) {
+    if (batch_div_on_tc(m, mv, shorts, sms)) {
         int c = 0;
         while (mv > 16u * DIV_TC_P[c] - (32u * DIV_TC_G[c] - 1) - 2) c++;
         return DIV_TC0 + c;
@@ -542,20 +549,33 @@ static size_t mul_smem_for(const bi_plan* p, int ipc_div) {
 // finely to the shifted inverse (15.9M -> 13.5M instances/s).  (Up to 128 limbs long division
 // stays: beside the batch's other kernels its small lane groups pack where
 // a CTA per division does not -- a 20000-instance batch ran 1.74 ms so and
-// 1.94 ms with the uniform entry's crossover.)  map[c] is the class that
-// size class c runs as.
+// 1.94 ms with the uniform entry's crossover.)
+struct DivMap {
+    uint64_t shorts = 0;          // see batch_div_on_tc
+    int sms = 0;
+    int to[DIV_CLASSES];          // the class that size class c runs as
+    int operator()(const bi_desc& d) const { return to[div_class(m64(d), mb64(d), shorts, sms)]; }
+};
+
 static uint32_t div_band(uint32_t max_mv) { return max_mv <= 256 ? 256 : max_mv <= 512 ? 512 : 1024; }
 
-static void div_class_map(const bi_desc* descs, const uint32_t* div, uint32_t n, int sms, int* map) {
+static DivMap div_class_map(const bi_desc* descs, const uint32_t* div, uint32_t n, int sms) {
     uint64_t cnt[DIV_CLASSES] = {};
     uint32_t max_m[DIV_CLASSES] = {};
+    DivMap map;
+    map.sms = sms;
     for (uint32_t k = 0; k < n; k++) {
-        const int c = div_class(m64(descs[div[k]]), mb64(descs[div[k]]));
+        const uint32_t mv = mb64(descs[div[k]]);
+        map.shorts += div_short_quotient(mv, m64(descs[div[k]]) - mv + 1, ~0ull, sms);
+    }
+    if (map.shorts <= 6 * (uint64_t)sms) map.shorts = 0;
+    for (uint32_t k = 0; k < n; k++) {
+        const int c = div_class(m64(descs[div[k]]), mb64(descs[div[k]]), map.shorts, sms);
         cnt[c]++;
         max_m[c] = std::max(max_m[c], m64(descs[div[k]]));
     }
     for (int c = 0; c < DIV_CLASSES; c++) {
-        map[c] = c;
+        map.to[c] = c;
         if (c >= DIV_THREAD_CLASSES && c < DIV_CTA_CLASS && max_m[c] <= BATCH_SHINV_MAX_M) {
             const uint32_t max_mv = DIV_WARP_CLASS_MAX_MV[c - DIV_THREAD_CLASSES];   // the class's largest divisor
             if (max_mv > 128) {
@@ -566,15 +586,16 @@ static void div_class_map(const bi_desc* descs, const uint32_t* div, uint32_t n,
                     if (bmv > 128 && div_band(bmv) == band) band_cnt += cnt[b];
                 }
                 const uint64_t per_sm = band == 256 ? 2 : band == 512 ? 3 : 6;
-                if (band_cnt <= per_sm * (uint64_t)sms) map[c] = DIV_CTA_CLASS;
+                if (band_cnt <= per_sm * (uint64_t)sms) map.to[c] = DIV_CTA_CLASS;
             }
         }
     }
+    return map;
 }
 
 // Division order: by class, then most expensive first.
-static bool div_before(const bi_desc& x, const bi_desc& y, const int* map) {
-    const int cx = map[div_class(m64(x), mb64(x))], cy = map[div_class(m64(y), mb64(y))];
+static bool div_before(const bi_desc& x, const bi_desc& y, const DivMap& map) {
+    const int cx = map(x), cy = map(y);
     if (cx != cy) return cx < cy;
     return (uint64_t)m64(x) * mb64(x) > (uint64_t)m64(y) * mb64(y);
 }
@@ -591,7 +612,7 @@ static size_t div_tc_smem(int k, uint32_t mu) {
     }
 }
 
-static void div_classes(bi_plan* p, const bi_desc* descs, const uint32_t* div, uint32_t n, const int* map) {
+static void div_classes(bi_plan* p, const bi_desc* descs, const uint32_t* div, uint32_t n, const DivMap& map) {
     p->div_smem = 0;
     for (uint32_t& mu : p->divc_mu) mu = 0;
     for (int c = 0; c < DIV_CLASSES; c++) {
@@ -601,7 +622,7 @@ static void div_classes(bi_plan* p, const bi_desc* descs, const uint32_t* div, u
     }
     for (uint32_t k = 0; k < n; k++) {
         const bi_desc& d = descs[div[k]];
-        const int c = map[div_class(m64(d), mb64(d))];
+        const int c = map(d);
         if (p->n_divc[c]++ == 0) p->div_off[c] = k;
         if (c == DIV_CTA_CLASS) p->divc_smem[c] = std::max(p->divc_smem[c], div_smem_bytes(div_geom(m64(d), mb64(d), 8)));
         if (c >= DIV_TC0) {
@@ -1006,8 +1027,7 @@ bi_status bi_plan_create(bi_plan** out_plan, const bi_desc* descs, uint64_t coun
     }
     // largest first: long instances start early, short ones fill the tail
     std::stable_sort(addsub.begin(), addsub.end(), [&](uint32_t x, uint32_t y) { return m64(descs[x]) > m64(descs[y]); });
-    int dmap[DIV_CLASSES];
-    div_class_map(descs, div.data(), (uint32_t)div.size(), num_sms(), dmap);
+    const DivMap dmap = div_class_map(descs, div.data(), (uint32_t)div.size(), num_sms());
     std::stable_sort(div.begin(), div.end(), [&](uint32_t x, uint32_t y) { return div_before(descs[x], descs[y], dmap); });
     std::stable_sort(mulkeys.begin(), mulkeys.end(), [](const std::pair<uint64_t, uint32_t>& x,
                                                         const std::pair<uint64_t, uint32_t>& y) {
@@ -1366,8 +1386,7 @@ extern "C" bi_status bi_batch_run_noalloc(const bi_desc* descs, uint64_t count, 
         }
     }
     std::stable_sort(na_add, na_add + na, [&](uint32_t x, uint32_t y) { return m64(descs[x]) > m64(descs[y]); });
-    int dmap[DIV_CLASSES];
-    div_class_map(descs, na_div, nd, num_sms(), dmap);
+    const DivMap dmap = div_class_map(descs, na_div, nd, num_sms());
     std::stable_sort(na_div, na_div + nd, [&](uint32_t x, uint32_t y) { return div_before(descs[x], descs[y], dmap); });
     std::stable_sort(na_keys, na_keys + nk, [](const std::pair<uint64_t, uint32_t>& x,
                                                const std::pair<uint64_t, uint32_t>& y) { return x.first > y.first; });

@@ -468,12 +468,21 @@ static bi_status div_tc(const T* u, const T* v, T* q, T* r, uint8_t* status, uin
 // 3399 / 626, 2000 6468 / 982).  With few instances the blocks' shorter chain
 // wins from about 20 quotient limbs on: 1 division of 2m by m limbs with m = 40
 // 20 / 13, 64 30 / 15, 256 83 / 26, 1024 360 / 89; 608 of them with m = 40 22 /
-// 18; 2432 with m = 72 61 / 54, with m = 64 50 / 54.
+// 18; 2432 with m = 72 61 / 54, with m = 64 50 / 54.  At two to four an SM it takes
+// a few more: 64 limbs by 20 quotient limbs, 304 divisions 10.2 / 10.3, 400 10.2 /
+// 11.3, 608 10.2 / 12.7 (by 24 11.7 / 12.5, by 40 17.6 / 15.4); 128 limbs by 20, 608
+// 12.2 / 12.8.  Four of more than 1024 limbs and few quotient limbs an SM are the
+// one full wave of CTAs that 8 quotient limbs at a time beat (1215 by 8: 608
+// divisions 28.7 / 35.8, 456 26.1 / 23.6, 760 57.0 / 39.4).
 static bool div_use_tc(uint32_t MU, uint32_t MV, uint64_t n) {
     const uint64_t ql = MU - MV + 1, sms = (uint64_t)num_sms();
     if (MV < 40 || MV > (uint32_t)DtShape<128, 1>::MAX_K) return false;
-    if (MV >= 65 && MV * ql >= 9400) return true;
-    return (ql >= 20 && n <= 4 * sms) || (MV >= 65 && ql >= 48 && n <= 16 * sms);
+    if (MV > 1024 && ql < 10 && n > 3 * sms && n <= 4 * sms) return false;
+    if (MV >= 65 && MV * ql >= 9400 && !div_short_quotient(MV, ql, n, (int)sms)) return true;
+    const bool few = n <= 2 * sms   ? ql >= 20
+                     : n <= 3 * sms ? ql >= (MV < 65 ? 24u : 20u)
+                                    : n <= 4 * sms && ql >= (MV < 65 ? 36u : 22u);
+    return few || (MV >= 65 && ql >= 48 && n <= 16 * sms);
 }
 
 // dividend limbs (u64 view) per instance: any long division, and the shifted inverse's limit

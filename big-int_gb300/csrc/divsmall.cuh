@@ -43,6 +43,20 @@ __host__ __device__ inline bool div_use_long(uint32_t MV, uint64_t n, int sms) {
     return n > per_sm * (uint64_t)sms;
 }
 
+// Divisors of 736 to 1024 limbs whose quotient (ql limbs) is too short for block
+// division (divtc.cuh) to earn back its setup against a warp's long division, n of
+// them (us, warps / blocks): 992 limbs, 4864 divisions: 12 quotient limbs 144 /
+// 231, 20 196 / 231, 24 221 / 230; 1216: 12 quotient limbs 38 / 58, 24 58 / 58;
+// 760: 10 quotient limbs 34 / 38, 14 40 / 38.  736 limbs, 4864: 14 quotient limbs
+// 108 / 127, 18 127 / 127; 2432: 14 61 / 59.  991 limbs, 2432: 12 72 / 78, 14 79 /
+// 78.  With fewer instances the shifted inverse stands in the warps' place, and
+// loses.
+__host__ inline bool div_short_quotient(uint32_t MV, uint64_t ql, uint64_t n, int sms) {
+    if (MV < 736 || MV > 1024) return false;
+    if (MV > 991) return n > 4 * (uint64_t)sms && ql < (n > 5 * (uint64_t)sms ? 26u : 14u);
+    return n > 5 * (uint64_t)sms && ql < (n > 16 * (uint64_t)sms ? 18u : 14u);
+}
+
 // Divisors of 17..128 limbs in a batch of at most DIV_SMALL_WARP_PER_SM
 // instances an SM divide on one warp each (div_warp with 1, 2 or 4 limbs a
 // lane) instead of sharing warps as lane groups: a warp's quotient limbs are

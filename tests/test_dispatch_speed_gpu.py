@@ -45,3 +45,43 @@ def test_sums_at_eight_words_stride(bigint, oracle, m):
     assert _us(lambda: B.add(a, b, out=r)) < (1.45 if m == 8 else 1.25) * ref
     k = slice(n - 50, n)
     assert (B.to_host(r[k], np.uint32) == oracle.add(B.to_host(a[k], np.uint32), B.to_host(b[k], np.uint32))).all()
+
+
+def _check_div(B, u, v, q, r, seed=0):
+    i = int(u.shape[0]) - 1
+    x, y = (int.from_bytes(t[i].cpu().numpy().tobytes(), "little") for t in (u, v))
+    assert tuple(int.from_bytes(t[i].cpu().numpy().tobytes(), "little") for t in (q, r)) == divmod(x, y)
+
+
+@pytest.mark.parametrize("mu,mv,n", [(83, 64, 608), (1003, 992, 4864), (1043, 1024, 2432), (749, 736, 9728), (1002, 991, 4864)])
+def test_divisions_with_short_quotients(bigint, mu, mv, n):
+    """Against long division on warps."""
+    import torch
+
+    B = bigint
+    u, v = _words(n, mu, 3, torch.int64), _words(n, mv, 4, torch.int64)
+    q, r, st = B.div(u, v)
+    _check_div(B, u, v, q, r)
+    long = _us(lambda: B.div(u, v, q=q, r=r, status=st, method="long"))
+    assert _us(lambda: B.div(u, v, q=q, r=r, status=st)) < 1.1 * long
+
+
+def test_plan_of_divisions_with_short_quotients(bigint):
+    """Many of them alone in a plan, against the uniform long division."""
+    import torch
+
+    B = bigint
+    mu, mv, n = 1003, 992, 4864
+    u, v = _words(n, mu, 5, torch.int64), _words(n, mv, 6, torch.int64)
+    arena = torch.cat([u.view(-1), v.view(-1)])
+    d = np.zeros(n, dtype=B.DESC_DTYPE)
+    i = np.arange(n, dtype=np.uint64)
+    d["op"], d["m"], d["mb"] = B.OP_DIV, mu, mv
+    d["a"], d["b"], d["r"], d["r2"], d["flag"] = i * mu, n * mu + i * mv, i * mu, n * mu + i * mv, i
+    out, fl = torch.zeros_like(arena), torch.zeros(n, dtype=torch.uint8, device="cuda")
+    plan = B.Plan(d, arena.numel(), arena.numel(), n)
+    t = _us(lambda: plan.execute(arena, out, fl))
+    q, r, st = B.div(u, v, method="long")
+    assert bool((out == torch.cat([q.view(-1), r.view(-1)])).all()) and bool((fl == st).all())
+    assert t < 1.2 * _us(lambda: B.div(u, v, q=q, r=r, status=st, method="long"))
+    plan.close()
