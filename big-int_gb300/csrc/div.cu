@@ -188,10 +188,21 @@ div_group_kernel(const T* __restrict__ u, const T* __restrict__ v, T* __restrict
 // for 15 by 7, 54 / 61 for 8 by 4.  Batches that do not fill the SMs have rows
 // at less latency: 50000 of 16 by 8 26.8 / 21.3, of 4 by 2 20.7 / 16.0.  Longer
 // rows leave too few warps an SM: u64 64 by 16 124 / 126 and 80 by 15 138 / 150,
-// u32 80 by 15 178 / 162.
+// u32 80 by 15 178 / 162.  Moving rows costs some 0.4 us, which few quotient limbs
+// do not earn back where the operands are in the L2 already (u64 5 by 4, 5000:
+// 2.9 / 3.4, 11 by 4 4.7 / 4.9, 20 by 4 7.3 / 7.3; 40000 of 11 by 4 6.6 / 7.5; 9 by 8,
+// 5000: 3.4 / 3.9, 20000: 4.6 / 4.6; u32 the same of 3-limb divisors, of 4-limb ones
+// by 2 3.3 / 3.7, by 6 5.1 / 4.9); with cold operands the two are equal there.
 constexpr int DIV_ROWS_PER_SM = 384;
 template <typename T>
 static bool div_thread_rows(uint32_t MU, uint32_t MV, uint64_t n, int sms) {
+    const uint32_t ql = MU - MV + 1;
+    const uint64_t per_sm = n / (uint64_t)sms;
+    if (MV < (sizeof(T) == 8 ? 8u : 4u)) {
+        if (ql < 8 || (ql < 24 && per_sm >= 160)) return false;
+    } else if (sizeof(T) == 8 ? ql < 8 && per_sm < 64 : MV < 8 && ql < 5 && per_sm < 160) {
+        return false;
+    }
     if (sizeof(T) == 4 && MV >= 4) return MU + MV <= 94;
     if (n <= (uint64_t)DIV_ROWS_PER_SM * (uint64_t)sms) return MU + MV <= 72;
     return sizeof(T) == 8 && MV >= 8 && MU <= 48;
