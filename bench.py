@@ -918,9 +918,11 @@ def run_single(args) -> None:
 
 
 def summary(extra, achieved_gbs: float, peak_gbs: float):
-    """The headline results of every workload in a few hundred bytes, the last
-    key of the JSON line: per size the instances/s and fraction of the
-    measured peak, and the ratios against the reference's own kernels."""
+    """The headline results of every workload in a few hundred bytes, beside
+    `extra`: per size the instances/s and fraction of the measured peak (the
+    integer pipe's also where the tensor cores do the work: above 1 there is
+    what that pipe alone could not do), and the ratios against the reference's
+    own kernels."""
     if not extra:
         return None
     sm = {"addsub_sweep_frac_of_hbm_peak": round(achieved_gbs / peak_gbs, 3)}
@@ -1148,9 +1150,11 @@ def run_ours(args) -> None:
                 "value": round(cpu_bytes / cpu_s / 1e9, 3), "unit": "GB/s", "cores": nthreads, "kind": "port",
                 "sample": f"the full sweep (same inputs, 2^27 limbs per size) run {cpu_reps}x: {cpu_s:.2f} s wall "
                           f"on {nthreads} threads; oracle port of ker-add.cu.h / sub.fut"},
-            "extra": extra,
-            "summary": summary(extra, achieved, peak),
         }
+        # the other workloads' rows (some 20 KB) apart, so that the line stays one
+        # that a log keeps whole
+        if extra:
+            print(json.dumps({"extra": extra, "summary": summary(extra, achieved, peak)}), file=sys.stderr, flush=True)
         print(json.dumps(line), flush=True)
     if world > 1:
         dist.destroy_process_group()
