@@ -27,7 +27,7 @@
 //     for a class above 128 limbs with too few divisions to fill the GPU,
 //     the crossover a uniform batch uses (div_use_long); divisors above 128
 //     limbs with quotients long enough to earn back the setup run 31 quotient
-//     limbs at a time on the tensor cores (divtc.cuh: the 20000-instance
+//     limbs (63 for divisors of 992 to 1215) at a time on the tensor cores (divtc.cuh: the 20000-instance
 //     batch's divisions alone 1345 -> 216 us, the 100000-instance batch's 3292
 //     -> 928); most expensive first within a class.
 // The persistent kernels run concurrently on forked streams; the fork,
@@ -227,8 +227,9 @@ constexpr int DIV_TC_P[DIV_TC_CLASSES] = {16, 32, 64, 80, 128};
 constexpr int DIV_TC_G[DIV_TC_CLASSES] = {1, 1, 1, 2, 1};   // as the uniform entry's for full batches
 constexpr int DIV_CLASSES = DIV_TC0 + DIV_TC_CLASSES;
 constexpr int DIV_CTA_THREADS = 512;
-// add/sub, multiply, one per division class, one per warp-multiply class
 constexpr int MUL_TC_CLASSES = 3;
+// add/sub, multiply, one per division class, warp-multiply class and tensor-core
+// multiply class
 constexpr int PLAN_KERNELS = 2 + DIV_CLASSES + MULW_CLASSES + MUL_TC_CLASSES;
 constexpr int PLAN_MULW0 = 2 + DIV_CLASSES;      // index of the first warp-multiply kernel
 constexpr int PLAN_MULTC0 = PLAN_MULW0 + MULW_CLASSES;   // and of the first tensor-core multiply kernel
@@ -263,8 +264,9 @@ static inline int div_class(uint32_t m, uint32_t mv, uint64_t shorts, int sms) {
 }
 
 // Multiplies on the tensor cores (multc.cuh) by the accumulator width that
-// holds the product: up to 512, 1024 and more product limbs.  The sizes are
-// the uniform entry's for batches that fill the GPU.
+// holds the product: up to 512, 1024 and more product limbs.  From the sizes on
+// at which they beat the batch's CTA kernel (the uniform entry, which has a warp
+// kernel below, goes there above 160 full and 256 truncated limbs).
 constexpr int MUL_TC_P[MUL_TC_CLASSES] = {32, 64, 128};
 constexpr uint32_t BATCH_TC_FULL_L = 160, BATCH_TC_TRUNC_L = 208;
 inline int multc_class(uint32_t m, bool full) {
@@ -600,7 +602,7 @@ static bool div_before(const bi_desc& x, const bi_desc& y, const DivMap& map) {
     return (uint64_t)m64(x) * mb64(x) > (uint64_t)m64(y) * mb64(y);
 }
 
-// Per-class offsets, counts and shared memory of a division list sorted by div_before.
+// Shared memory of tensor-core class k with dividends of up to mu limbs.
 static size_t div_tc_smem(int k, uint32_t mu) {
     const DtGeom g = dt_geom(mu, 1, 8);
     switch (k) {
@@ -612,6 +614,7 @@ static size_t div_tc_smem(int k, uint32_t mu) {
     }
 }
 
+// Per-class offsets, counts and shared memory of a division list sorted by div_before.
 static void div_classes(bi_plan* p, const bi_desc* descs, const uint32_t* div, uint32_t n, const DivMap& map) {
     p->div_smem = 0;
     for (uint32_t& mu : p->divc_mu) mu = 0;

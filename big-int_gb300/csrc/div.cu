@@ -399,7 +399,7 @@ static void launch_div_blk(const T* u, const T* v, T* q, T* r, uint8_t* status, 
 // divisions of 2048 by 1024 limbs 3400 -> 565 us, 8192 of 512 by 256 1013 ->
 // 409.  Bound by the latency of a block's chain -- estimate, product, fold,
 // carries, each behind a barrier: issue slots 45 % busy at four CTAs an SM (what
-// tensor memory holds at 1024 limbs), the tensor core about 40 %.
+// tensor memory holds at 1024 limbs), the tensor core 30 %.
 // ---------------------------------------------------------------------------
 // (P = 16 held to 12 CTAs an SM, 40 registers: 192-limb divisors 376 -> 347 us at
 // 10922, 128-limb ones 418 -> 403; wider shapes ran slower so.  0 leaves the bound to

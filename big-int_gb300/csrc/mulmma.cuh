@@ -190,7 +190,7 @@ __device__ __forceinline__ void mm_product(const Item& it, const MmLimbs<MmShape
     // ldmatrix: rows lane & 7 of the four 8 x 8 parts (rows 0.., rows 8.., then the same 8 digits on)
     const uint32_t ap = (uint32_t)__cvta_generic_to_shared(a16) +
                         16 * ((lane & 7) + ((lane >> 3) & 1) * 8) + 16 * (lane >> 4);
-    {   // r = 0, w = 0: before the move below, so that both halves hold at most 1024 products a column
+    auto first_tile = [&] {   // r = 0, w = 0
         const uint32_t b0 = bp[0], b1 = bp[-4];
 #pragma unroll
         for (int v = 0; v < (FULL ? LT + 1 : LT); v++) {
@@ -198,7 +198,11 @@ __device__ __forceinline__ void mm_product(const Item& it, const MmLimbs<MmShape
             mm_ldmatrix(a, ap + 256 * v);
             mm_mma(c[v], a, b0, b1);
         }
-    }
+    };
+    // before the move below, so that both halves hold at most 1024 products a
+    // column; where there is none it comes last (first it cost full products of 113
+    // to 128 limbs 6 %)
+    if (S::FLUSH) first_tile();
     // (all residues unrolled run 8-10 % faster up to 64 limbs, slower above)
 #pragma unroll (LT <= 5 ? 8 : 1)
     for (int r = 0; r < 8; r++) {
@@ -232,6 +236,7 @@ __device__ __forceinline__ void mm_product(const Item& it, const MmLimbs<MmShape
                 }
         }
     }
+    if (!S::FLUSH) first_tile();
     __syncwarp();   // the operands are read
 
     // ---- sums to the lanes that own their limbs: limb l's eight in lane l / O
