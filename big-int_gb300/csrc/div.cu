@@ -403,9 +403,12 @@ static void launch_div_blk(const T* u, const T* v, T* q, T* r, uint8_t* status, 
 // ---------------------------------------------------------------------------
 // (P = 16 held to 12 CTAs an SM, 40 registers: 192-limb divisors 376 -> 347 us at
 // 10922, 128-limb ones 418 -> 403; wider shapes ran slower so.  0 leaves the bound to
-// the compiler, 64 to 96 registers; a 1 lets it take 250: 1024 limbs 565 -> 930 us)
+// the compiler, 64 to 96 registers; a 1 lets it take 250: 1024 limbs 565 -> 930 us.
+// P = 64 at 7, 72 registers: at the compiler's 64 it spills, 2849 divisions of 1472
+// by 736 limbs 521 -> 500 us, 2116 of 1982 by 991 551 -> 523; shared memory holds
+// four or five CTAs there)
 template <typename T, int P, int G, uint32_t HELD = 0>
-__global__ void __launch_bounds__(DtShape<P, G>::NT, P == 16 ? 12 : 0)
+__global__ void __launch_bounds__(DtShape<P, G>::NT, P == 16 ? 12 : P == 64 ? 7 : 0)
 div_tc_kernel(const T* __restrict__ u, const T* __restrict__ v, T* __restrict__ q, T* __restrict__ r,
               uint8_t* __restrict__ status, uint64_t n, DtGeom g, uint32_t* gave_up) {
     extern __shared__ __align__(128) uint8_t smem_dt[];
