@@ -178,9 +178,9 @@ bi_status bi_div_u32(const uint32_t* u, const uint32_t* v, uint32_t* q, uint32_t
 /* not: q and r are unique): schoolbook long division on one thread per     */
 /* instance up to 16 divisor limbs and on one warp or lane group (8 or 16   */
 /* lanes, 1 to 32 limbs a lane) per instance up to 1024 limbs; long         */
-/* division 31 quotient limbs at a time on the tensor cores for divisors of */
-/* 40 (small batches) or 65 up to 2015 limbs once the quotient is long      */
-/* enough to earn back its setup; above that 8 quotient limbs at a time on  */
+/* division 31 or 63 quotient limbs at a time on the tensor cores for       */
+/* divisors of 40 (small batches) or 65 up to 2015 limbs once the quotient  */
+/* is long enough to earn back its setup; above that 8 quotient limbs at a time on  */
 /* four warps; the shifted inverse for few divisions with short quotients.  */
 /* The _shinv entries take the shifted inverse at every size (the         */
 /* reference's algorithm; dividends up to 2048 64-bit limbs, else         */
